@@ -455,7 +455,8 @@ KERNEL_GEOMETRY = {
     "dense_ffn_mma_kernel": {"block": 512, "grid_barriers": 1, "max_tokens": 8},
     "attention_decode_stream_kernel": {"block": 288, "grid_barriers": 1},
     "dense_ffn_stream_kernel": {"block": 416, "grid_barriers": 1, "max_tokens": 1},
-    "linear_attention_kernel": {"block": 256, "grid_barriers": 0},
+    "linear_attention_kernel": {"block": 256, "grid_barriers": 0},  # unaligned shapes only
+    "linear_strip_kernel": {"block": 64, "grid_barriers": 0},
     "linear_decode_kernel": {"block": 288, "grid_barriers": 0, "max_tokens": 8},
 }
 _SMEM_OPTIN = 232448   # bytes of shared memory one CTA may use on sm_100
@@ -536,8 +537,8 @@ def _kernel_schedule(graph: TaskGraph, wc: WorkerConfig, batch: int, context_len
             dk, dv = cfg.linear_key_head_dim, cfg.linear_value_head_dim
             launches.append(KernelLaunch(
                 name=f"layer_{li}_linear_attention", entry_point="mk36_linear_attention_decode", task_ids=(task.id,),
-                kernel="linear_attention_kernel", grid=batch * hv * _ceil_div(dv, 32),
-                block=KERNEL_GEOMETRY["linear_attention_kernel"]["block"], grid_barriers=0, layer=li,
+                kernel="linear_strip_kernel", grid=batch * hv * _ceil_div(dv, 32),
+                block=KERNEL_GEOMETRY["linear_strip_kernel"]["block"], grid_barriers=0, layer=li,
                 phases=(KernelPhase("state_update_and_readout", batch * hv * dk, dv * 4 * 2, "static"),),
                 hbm_bytes=2 * batch * hv * dk * dv * 4 + batch * (2 * hk * dk + 2 * hv * dv) * 2))
         elif task.kind == "rmsnorm" and (task.id.endswith("_attn_norm") or task.id == "final_norm"):
