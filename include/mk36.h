@@ -245,6 +245,40 @@ MK36_API size_t mk36_attention_workspace_bytes(const mk36_attention_args* args);
 MK36_API int mk36_full_attention_decode(const mk36_attention_args* args, void* workspace,
                                         size_t workspace_bytes, void* stream);
 
+/* The same over caches whose batch items lie `cache_batch_stride` elements apart (0: dense): the first seq_len
+ * tokens of caches [batch, capacity, kv_heads, head_dim] with capacity * kv_heads * head_dim as the stride.  No
+ * counterpart in the reference (its caches are as long as the context). */
+MK36_API int mk36_full_attention_decode_strided(const mk36_attention_args* args, int64_t cache_batch_stride, void* workspace,
+                                                size_t workspace_bytes, void* stream);
+
+/* ---------------------------------------------------------------------------------------------
+ * The step between a q | k | v projection and attention: rotate-half rotary embedding of the new
+ * token's query and key on the first rotary_dim channels (mega_kernel_qwen36/reference.py:91-114;
+ * skipped when cos is NULL) and the append of its key and value at `position` of the caches.
+ *
+ * Layouts: qkv [batch, (query_heads + 2 kv_heads) * head_dim], rows of the query heads, the key heads, the
+ * value heads; cos, sin fp32 [rotary_dim]; q (output) [batch, query_heads, head_dim]; k_cache, v_cache
+ * [batch, capacity, kv_heads, head_dim], written at `position`.  No workspace is needed.
+ * ------------------------------------------------------------------------------------------ */
+typedef struct mk36_attention_append_args {
+    const void* qkv;
+    const float* cos;
+    const float* sin;
+    void* q;
+    void* k_cache;
+    void* v_cache;
+    int32_t dtype; /* of qkv, q and the caches */
+    int32_t batch;
+    int32_t query_heads;
+    int32_t kv_heads;
+    int32_t head_dim;
+    int32_t rotary_dim;
+    int64_t position;
+    int64_t capacity;
+} mk36_attention_append_args;
+
+MK36_API int mk36_attention_append(const mk36_attention_append_args* args, void* stream);
+
 /* Full-attention decode for callers that cannot provide a workspace.  This entry point has no
  * counterpart in the reference: it exists for hosts that bind the library over a plain C boundary
  * and own no device allocator, or that sit in a request loop where cudaMalloc / cudaFree (which

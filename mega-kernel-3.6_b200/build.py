@@ -37,6 +37,7 @@ CUDA_SOURCES = [
     "dense_ffn_decode.cu",
     "dense_ffn_mma.cu",
     "dense_ffn_stream.cu",
+    "attention_append.cu",
     "attention_decode.cu",
     "attention_decode_mma.cu",
     "attention_decode_stream.cu",

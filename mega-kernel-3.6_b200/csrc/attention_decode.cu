@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kAttnThreads) attention_decode_generic_kernel(
     }
 
     const size_t tok_stride = (size_t)p.Hkv * p.D;
-    const size_t base = (size_t)b * p.T * tok_stride + (size_t)kvh * p.D;
+    const size_t base = (size_t)b * p.kv_stride + (size_t)kvh * p.D;
     for (int t = t_begin + warp; t < t_end; t += kAttnWarps) {
         const T* kr = kc + base + (size_t)t * tok_stride;
         const T* vr = vc + base + (size_t)t * tok_stride;
@@ -191,19 +191,23 @@ void plan_generic(const mk36_attention_args& a, int max_ctas, AttnPlan* plan) {
 
 }  // namespace
 
-int attention_decode_mma_launch(const mk36_attention_args* a, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool* handled);
-int attention_decode_stream_launch(const mk36_attention_args* a, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool* handled);
+int attention_decode_mma_launch(const mk36_attention_args* a, size_t kv_stride, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool* handled);
+int attention_decode_stream_launch(const mk36_attention_args* a, size_t kv_stride, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool* handled);
 
-int attention_decode_launch(const mk36_attention_args* a, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+// kv_stride: elements from one batch item's cache to the next (0: dense)
+int attention_decode_launch(const mk36_attention_args* a, size_t kv_stride, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
     int rc = check_attention_args(a);
     if (rc != MK36_OK) return rc;
+    const size_t dense = (size_t)a->seq_len * a->kv_heads * a->head_dim;
+    if (kv_stride == 0) kv_stride = dense;
+    if (kv_stride < dense) MK36_FAIL(MK36_ERR_INVALID_ARG, "full_attention_decode: the cache's batch stride is smaller than its tokens");
     if (!options().force_generic) {
         bool handled = false;
         if (options().attn_stream) {
-            rc = attention_decode_stream_launch(a, workspace, workspace_bytes, stream, &handled);
+            rc = attention_decode_stream_launch(a, kv_stride, workspace, workspace_bytes, stream, &handled);
             if (rc != MK36_OK || handled) return rc;
         }
-        rc = attention_decode_mma_launch(a, workspace, workspace_bytes, stream, &handled);
+        rc = attention_decode_mma_launch(a, kv_stride, workspace, workspace_bytes, stream, &handled);
         if (rc != MK36_OK || handled) return rc;
     }
     const DeviceInfo* dev = current_device_info();
@@ -248,8 +252,8 @@ int attention_decode_launch(const mk36_attention_args* a, void* workspace, size_
         plan_generic(sub, (int)max_ctas, &plan);
         AttnParams p;
         p.q = static_cast<const unsigned char*>(a->q) + (size_t)b0 * a->query_heads * a->head_dim * es;
-        p.k = static_cast<const unsigned char*>(a->k_cache) + (size_t)b0 * a->seq_len * a->kv_heads * a->head_dim * es;
-        p.v = static_cast<const unsigned char*>(a->v_cache) + (size_t)b0 * a->seq_len * a->kv_heads * a->head_dim * es;
+        p.k = static_cast<const unsigned char*>(a->k_cache) + (size_t)b0 * kv_stride * es;
+        p.v = static_cast<const unsigned char*>(a->v_cache) + (size_t)b0 * kv_stride * es;
         p.out = static_cast<unsigned char*>(a->out) + (size_t)b0 * a->query_heads * a->head_dim * es;
         p.ctl = static_cast<Control*>(workspace);
         unsigned char* scratch = static_cast<unsigned char*>(workspace) + kControlBytes;
@@ -264,6 +268,7 @@ int attention_decode_launch(const mk36_attention_args* a, void* workspace, size_
         p.Hkv = a->kv_heads;
         p.D = a->head_dim;
         p.T = a->seq_len;
+        p.kv_stride = kv_stride;
         p.group = group;
         p.subgroups = plan.subgroups;
         p.splits = plan.splits;
@@ -291,7 +296,13 @@ size_t mk36_attention_workspace_bytes(const mk36_attention_args* a) {
 }
 
 int mk36_full_attention_decode(const mk36_attention_args* args, void* workspace, size_t workspace_bytes, void* stream) {
-    return attention_decode_launch(args, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+    return attention_decode_launch(args, 0, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+int mk36_full_attention_decode_strided(const mk36_attention_args* args, int64_t cache_batch_stride, void* workspace, size_t workspace_bytes,
+                                       void* stream) {
+    if (cache_batch_stride < 0) MK36_FAIL(MK36_ERR_INVALID_ARG, "full_attention_decode: the cache's batch stride is negative");
+    return attention_decode_launch(args, (size_t)cache_batch_stride, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(kMmaAttnThreads, 1) attention_decode_mma_kerne
     const int tile_end = (int)(((long long)tiles_total * (split + 1)) / p.splits);
 
     const size_t tok_stride = (size_t)p.Hkv * D;  // elements between consecutive tokens
-    const T* kbase = static_cast<const T*>(p.k) + (size_t)b * p.T * tok_stride + (size_t)kvh * D;
-    const T* vbase = static_cast<const T*>(p.v) + (size_t)b * p.T * tok_stride + (size_t)kvh * D;
+    const T* kbase = static_cast<const T*>(p.k) + (size_t)b * p.kv_stride + (size_t)kvh * D;
+    const T* vbase = static_cast<const T*>(p.v) + (size_t)b * p.kv_stride + (size_t)kvh * D;
 
     float o[NW][4];
 #pragma unroll
@@ -303,7 +303,7 @@ const void* mma_kernel_for(int d) {
 
 // Launches the tensor-core variant when the shapes suit it and sets *handled; otherwise leaves
 // *handled false (no error) and the caller uses the general kernel.
-int attention_decode_mma_launch(const mk36_attention_args* a, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool* handled) {
+int attention_decode_mma_launch(const mk36_attention_args* a, size_t kv_stride, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool* handled) {
     *handled = false;
     if (a->dtype != MK36_BF16 && a->dtype != MK36_F16) return MK36_OK;
     const int D = a->head_dim, group = a->query_heads / a->kv_heads;
@@ -311,6 +311,7 @@ int attention_decode_mma_launch(const mk36_attention_args* a, void* workspace, s
     const void* ptrs[] = {a->q, a->k_cache, a->v_cache};
     for (const void* q : ptrs)
         if ((reinterpret_cast<uintptr_t>(q) & 15u) != 0) return MK36_OK;
+    if (kv_stride % 8 != 0) return MK36_OK;
     const DeviceInfo* dev = current_device_info();
     if (!dev) return MK36_ERR_LAUNCH;
     const void* kernel = (a->dtype == MK36_BF16) ? mma_kernel_for<__nv_bfloat16>(D) : mma_kernel_for<__half>(D);
@@ -353,8 +354,8 @@ int attention_decode_mma_launch(const mk36_attention_args* a, void* workspace, s
         const size_t heads = (size_t)nb * a->query_heads;
         AttnParams p;
         p.q = static_cast<const unsigned char*>(a->q) + (size_t)b0 * a->query_heads * D * es;
-        p.k = static_cast<const unsigned char*>(a->k_cache) + (size_t)b0 * a->seq_len * a->kv_heads * D * es;
-        p.v = static_cast<const unsigned char*>(a->v_cache) + (size_t)b0 * a->seq_len * a->kv_heads * D * es;
+        p.k = static_cast<const unsigned char*>(a->k_cache) + (size_t)b0 * kv_stride * es;
+        p.v = static_cast<const unsigned char*>(a->v_cache) + (size_t)b0 * kv_stride * es;
         p.out = static_cast<unsigned char*>(a->out) + (size_t)b0 * a->query_heads * D * es;
         p.ctl = static_cast<Control*>(workspace);
         unsigned char* sc = static_cast<unsigned char*>(workspace) + kControlBytes;
@@ -368,6 +369,7 @@ int attention_decode_mma_launch(const mk36_attention_args* a, void* workspace, s
         p.Hkv = a->kv_heads;
         p.D = D;
         p.T = a->seq_len;
+        p.kv_stride = kv_stride;
         p.group = group;
         p.subgroups = 1;
         p.splits = (int)splits;

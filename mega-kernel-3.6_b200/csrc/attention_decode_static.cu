@@ -35,7 +35,7 @@
 
 namespace mk36 {
 
-int attention_decode_launch(const mk36_attention_args* a, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+int attention_decode_launch(const mk36_attention_args* a, size_t kv_stride, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
 namespace {
 
@@ -93,7 +93,7 @@ int mk36_full_attention_decode_static(const mk36_attention_args* args, void* str
     // lets a test lower it so that the refusal can be exercised with a small problem)
     size_t limit = kStaticScratchBytes;
     if (options().static_scratch_limit > 0 && (size_t)options().static_scratch_limit < limit) limit = (size_t)options().static_scratch_limit;
-    rc = attention_decode_launch(args, scratch, limit, s);
+    rc = attention_decode_launch(args, 0, scratch, limit, s);
     if (rc == MK36_ERR_WORKSPACE) {
         MK36_FAIL(MK36_ERR_WORKSPACE,
                   "full_attention_decode_static: batch %d x %d query heads x head_dim %d at %d cached tokens needs more scratch than the "

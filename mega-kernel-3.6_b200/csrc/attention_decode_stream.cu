@@ -141,8 +141,8 @@ __global__ void __launch_bounds__(kAsThreads, 1) attention_decode_stream_kernel(
             *(volatile int*)&s_abort = 1;
             return;
         }
-        const T* kbase = static_cast<const T*>(p.k) + (size_t)b * p.T * tok_elems;
-        const T* vbase = static_cast<const T*>(p.v) + (size_t)b * p.T * tok_elems;
+        const T* kbase = static_cast<const T*>(p.k) + (size_t)b * p.kv_stride;
+        const T* vbase = static_cast<const T*>(p.v) + (size_t)b * p.kv_stride;
         bool ok = true;
         int stage = 0, use = 0;
         // the first rounds are dealt statically (chunk k * splits + split), the rest through the counter
@@ -413,7 +413,7 @@ const void* stream_kernel_for(int d) {
 
 // Launches the streaming variant when the shapes suit it and sets *handled; otherwise leaves *handled false
 // (no error) and the caller tries the other kernels.
-int attention_decode_stream_launch(const mk36_attention_args* a, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool* handled) {
+int attention_decode_stream_launch(const mk36_attention_args* a, size_t kv_stride, void* workspace, size_t workspace_bytes, cudaStream_t stream, bool* handled) {
     *handled = false;
     if (a->dtype != MK36_BF16 && a->dtype != MK36_F16) return MK36_OK;
     const int D = a->head_dim, Hkv = a->kv_heads, group = a->query_heads / a->kv_heads;
@@ -425,6 +425,7 @@ int attention_decode_stream_launch(const mk36_attention_args* a, void* workspace
     const void* ptrs[] = {a->q, a->k_cache, a->v_cache};
     for (const void* q : ptrs)
         if ((reinterpret_cast<uintptr_t>(q) & 15u) != 0) return MK36_OK;
+    if (kv_stride % 8 != 0) return MK36_OK;
     const DeviceInfo* dev = current_device_info();
     if (!dev) return MK36_ERR_LAUNCH;
     const void* kernel = (a->dtype == MK36_BF16) ? stream_kernel_for<__nv_bfloat16>(D) : stream_kernel_for<__half>(D);
@@ -485,8 +486,8 @@ int attention_decode_stream_launch(const mk36_attention_args* a, void* workspace
         const size_t heads = (size_t)nb * a->query_heads;
         AttnParams& p = sp.a;
         p.q = static_cast<const unsigned char*>(a->q) + (size_t)b0 * a->query_heads * D * es;
-        p.k = static_cast<const unsigned char*>(a->k_cache) + (size_t)b0 * a->seq_len * Hkv * D * es;
-        p.v = static_cast<const unsigned char*>(a->v_cache) + (size_t)b0 * a->seq_len * Hkv * D * es;
+        p.k = static_cast<const unsigned char*>(a->k_cache) + (size_t)b0 * kv_stride * es;
+        p.v = static_cast<const unsigned char*>(a->v_cache) + (size_t)b0 * kv_stride * es;
         p.out = static_cast<unsigned char*>(a->out) + (size_t)b0 * a->query_heads * D * es;
         p.ctl = static_cast<Control*>(workspace);
         unsigned char* sc = static_cast<unsigned char*>(workspace) + kControlBytes;
@@ -500,6 +501,7 @@ int attention_decode_stream_launch(const mk36_attention_args* a, void* workspace
         p.Hkv = Hkv;
         p.D = D;
         p.T = a->seq_len;
+        p.kv_stride = kv_stride;
         p.group = group;
         p.subgroups = 1;
         p.splits = (int)splits;

@@ -16,6 +16,7 @@ struct AttnParams {
     float* part_o;  // [B][Hq][splits][D]
     float* part_m;  // [B][Hq][splits]
     float* part_l;  // [B][Hq][splits]
+    size_t kv_stride;  // elements from one batch item's cache to the next
     int B, Hq, Hkv, D, T;
     int group;      // Hq / Hkv
     int subgroups;  // CTAs that share one KV head's stream because a CTA serves at most GP heads

@@ -407,6 +407,69 @@ torch::Tensor full_attention_decode(torch::Tensor q, torch::Tensor k_cache, torc
 }
 
 // -------------------------------------------------------------------------------------------
+// A full-attention block with its projections: four launches and no tensor operation between them.  cos / sin:
+// fp32 [rotary_dim] on the device.  Writes the caches at `position`; returns (out, attention output).
+// -------------------------------------------------------------------------------------------
+std::tuple<torch::Tensor, torch::Tensor> attention_block_decode(torch::Tensor hidden, torch::Tensor norm_weight, torch::Tensor qkv_weight,
+                                                                torch::Tensor out_weight, torch::Tensor k_cache, torch::Tensor v_cache,
+                                                                int64_t position, int64_t query_heads, int64_t kv_heads, int64_t head_dim,
+                                                                c10::optional<torch::Tensor> cos, c10::optional<torch::Tensor> sin,
+                                                                double scale, double eps) {
+    SHIM_CHECK_INPUT(k_cache);
+    SHIM_CHECK_INPUT(v_cache);
+    const int64_t batch = hidden.size(0);
+    TORCH_CHECK(k_cache.dim() == 4 && k_cache.size(0) == batch && k_cache.size(2) == kv_heads && k_cache.size(3) == head_dim,
+                "k_cache must be [batch, capacity, kv_heads, head_dim]");
+    TORCH_CHECK(v_cache.sizes() == k_cache.sizes(), "v_cache shape must match k_cache");
+    TORCH_CHECK(hidden.scalar_type() == k_cache.scalar_type(), "q and k_cache dtype mismatch");
+    TORCH_CHECK(hidden.scalar_type() == v_cache.scalar_type(), "q and v_cache dtype mismatch");
+    TORCH_CHECK(query_heads % kv_heads == 0, "query_heads must be divisible by kv_heads");
+    TORCH_CHECK(head_dim <= 256, "head_dim > 256 is not supported by this kernel");
+    const c10::cuda::CUDAGuard guard(hidden.device());
+    torch::Tensor qkv = std::get<0>(linear_decode(hidden, qkv_weight, norm_weight, c10::nullopt, eps, false));
+    torch::Tensor q = torch::empty({batch, query_heads, head_dim}, hidden.options());
+    torch::Tensor attn = torch::empty_like(q);
+    mk36_attention_append_args ap{};
+    ap.qkv = qkv.data_ptr();
+    if (cos.has_value()) {
+        TORCH_CHECK(cos->is_cuda() && cos->is_contiguous() && cos->scalar_type() == torch::kFloat32 && sin.has_value() && sin->is_cuda() &&
+                        sin->is_contiguous() && sin->scalar_type() == torch::kFloat32 && sin->numel() == cos->numel(),
+                    "cos and sin must be contiguous float32 CUDA tensors of one length");
+        ap.cos = cos->data_ptr<float>();
+        ap.sin = sin->data_ptr<float>();
+        ap.rotary_dim = static_cast<int32_t>(cos->numel());
+    }
+    ap.q = q.data_ptr();
+    ap.k_cache = k_cache.data_ptr();
+    ap.v_cache = v_cache.data_ptr();
+    ap.dtype = dtype_code(hidden, "attention_block_decode");
+    ap.batch = static_cast<int32_t>(batch);
+    ap.query_heads = static_cast<int32_t>(query_heads);
+    ap.kv_heads = static_cast<int32_t>(kv_heads);
+    ap.head_dim = static_cast<int32_t>(head_dim);
+    ap.position = position;
+    ap.capacity = k_cache.size(1);
+    const auto stream = at::cuda::getCurrentCUDAStream().stream();
+    check_rc(mk36_attention_append(&ap, stream));
+    mk36_attention_args a{};
+    a.q = ap.q;
+    a.k_cache = ap.k_cache;
+    a.v_cache = ap.v_cache;
+    a.out = attn.data_ptr();
+    a.dtype = ap.dtype;
+    a.batch = ap.batch;
+    a.query_heads = ap.query_heads;
+    a.kv_heads = ap.kv_heads;
+    a.head_dim = ap.head_dim;
+    a.seq_len = static_cast<int32_t>(position + 1);
+    a.scale = static_cast<float>(scale);
+    Workspace& ws = workspace_for(q, mk36_attention_workspace_bytes(&a));
+    check_rc(mk36_full_attention_decode_strided(&a, ap.capacity * kv_heads * head_dim, ws.buffer.data_ptr(), ws.bytes, stream));
+    torch::Tensor out = std::get<0>(linear_decode(attn.view({batch, query_heads * head_dim}), out_weight, c10::nullopt, hidden, 0.0, false));
+    return {out, attn};
+}
+
+// -------------------------------------------------------------------------------------------
 // linear_attention_decode: same name, arguments and return value as csrc/bindings.cpp:35.
 // linear_attention_decode_ex adds per-(batch, head) decay / beta, grouped key heads and an
 // optional in-place state update.
@@ -569,6 +632,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("ipc_close", &ipc_close);
     m.def("linear_decode", &linear_decode, "decode-time projection with optional fused RMSNorm, residual and arg-max (sm_100a)");
     m.def("full_attention_decode", &full_attention_decode, "Qwen3.6 full-attention decode kernel (sm_100a)");
+    m.def("attention_block_decode", &attention_block_decode, "norm + q|k|v projection, rotary, cache append, attention, output projection");
     m.def("linear_attention_decode", &linear_attention_decode, "Qwen3.6 linear-attention recurrent decode kernel (sm_100a)");
     m.def("linear_attention_decode_ex", &linear_attention_decode_ex, "per-head decay/beta, grouped keys, optional in-place state",
           py::arg("q"), py::arg("k"), py::arg("v"), py::arg("state"), py::arg("decay") = 1.0,

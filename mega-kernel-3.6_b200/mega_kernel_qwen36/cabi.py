@@ -60,6 +60,14 @@ class AttentionArgs(C.Structure):
     ]
 
 
+class AttentionAppendArgs(C.Structure):
+    _fields_ = [
+        ("qkv", C.c_void_p), ("cos", C.c_void_p), ("sin", C.c_void_p), ("q", C.c_void_p), ("k_cache", C.c_void_p), ("v_cache", C.c_void_p),
+        ("dtype", C.c_int32), ("batch", C.c_int32), ("query_heads", C.c_int32), ("kv_heads", C.c_int32), ("head_dim", C.c_int32),
+        ("rotary_dim", C.c_int32), ("position", C.c_int64), ("capacity", C.c_int64),
+    ]
+
+
 class LinearAttentionArgs(C.Structure):
     _fields_ = [
         ("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("state", C.c_void_p),
@@ -107,6 +115,8 @@ SIGNATURES = {
     "mk36_linear_decode": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p, C.c_size_t, C.c_void_p]),
     "mk36_attention_workspace_bytes": (C.c_size_t, [C.POINTER(AttentionArgs)]),
     "mk36_full_attention_decode": (C.c_int, [C.POINTER(AttentionArgs), C.c_void_p, C.c_size_t, C.c_void_p]),
+    "mk36_full_attention_decode_strided": (C.c_int, [C.POINTER(AttentionArgs), C.c_int64, C.c_void_p, C.c_size_t, C.c_void_p]),
+    "mk36_attention_append": (C.c_int, [C.POINTER(AttentionAppendArgs), C.c_void_p]),
     "mk36_full_attention_decode_static": (C.c_int, [C.POINTER(AttentionArgs), C.c_void_p]),
     "mk36_static_scratch_status": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
     "mk36_linear_attention_decode": (C.c_int, [C.POINTER(LinearAttentionArgs), C.c_void_p]),

@@ -246,14 +246,32 @@ def full_attention_decode(inputs: FullAttentionInputs) -> torch.Tensor:
 def attention_block_decode(hidden: torch.Tensor, block: AttentionBlockInputs, *, eps: float = 1e-6) -> Tuple[torch.Tensor, torch.Tensor]:
     """hidden [B, H] -> (hidden + out_proj(attention(q, cache)), attention output [B, Hq, D]).
 
-    Three launches: the fused RMSNorm + q|k|v projection, the attention kernel over the cache including
-    the new token, and the output projection with the residual added before the single rounding."""
+    Four launches: the fused RMSNorm + q|k|v projection, rotary embedding + cache append, the attention
+    kernel over the cache including the new token, and the output projection with the residual added
+    before the single rounding.  Attention reads the caches where they lie, whatever their capacity."""
     hq, hkv, d = block.query_heads, block.kv_heads, block.head_dim
     b = hidden.shape[0]
     if block.qkv_weight.shape[0] != (hq + 2 * hkv) * d:
         raise ValueError("qkv_weight must have (query_heads + 2 * kv_heads) * head_dim rows")
     if not 0 <= block.position < block.k_cache.shape[1]:
         raise ValueError("position must lie inside the cache")
+    cos, sin = block.cos, block.sin
+    if cos is None or sin is None or block.rotary_dim <= 0:
+        cos = sin = None
+    k_cache, v_cache = block.k_cache, block.v_cache
+    if (
+        block.input_norm_weight is not None and k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.shape == v_cache.shape == (b, k_cache.shape[1], hkv, d)
+        and hidden.dtype == k_cache.dtype == v_cache.dtype and hidden.device == k_cache.device == v_cache.device
+        and (cos is None or (cos.numel() == sin.numel() == cos.shape[-1] == sin.shape[-1] == block.rotary_dim <= d))
+    ):
+        ext = _native("attention_block_decode", hidden, k_cache, v_cache, block.qkv_weight, block.out_weight, block.input_norm_weight)
+        if cos is not None:
+            cos = cos.to(device=hidden.device, dtype=torch.float32).reshape(-1)
+            sin = sin.to(device=hidden.device, dtype=torch.float32).reshape(-1)
+        scale = 1.0 / math.sqrt(d) if block.scale is None else block.scale
+        return ext.attention_block_decode(hidden, block.input_norm_weight, block.qkv_weight, block.out_weight, k_cache, v_cache,
+                                          block.position, hq, hkv, d, cos, sin, float(scale), float(eps))
+    # caches that are views, or cos / sin of another form: the same steps as tensor operations
     qkv = linear_decode(hidden, block.qkv_weight, norm_weight=block.input_norm_weight, eps=eps)
     q = qkv[:, : hq * d].reshape(b, hq, d)
     k_new = qkv[:, hq * d : (hq + hkv) * d].reshape(b, 1, hkv, d)
