@@ -89,7 +89,8 @@ MK36_API int mk36_workspace_status(void* workspace, void* stream, int* device_st
  * batch kernel, eight tokens per launch (one grid barrier, the same weight stream).  "moe_stream"
  * is the largest token count the stream kernel takes (default 1; 2 also sends two-token calls to
  * it, 0 none); "moe_batch" = 0 sends what the stream kernel does not take to the ring kernel
- * instead of the batch kernel; "ring_mma" = 1 additionally makes the ring kernel contract with
+ * instead of the batch kernel (and the wide kernel); "moe_wide" is the smallest token count for which bf16 calls
+ * run the wide kernel, 32 tokens per launch with every distinct expert read once (default 9, 0 = never); "ring_mma" = 1 additionally makes the ring kernel contract with
  * tensor-core instructions whatever the token count.  "moe_stages" (0 = default, else 2..6) sets the stream and
  * batch kernels' ring depth, "moe_static" = 1 makes them (and the dense streaming kernel) deal
  * chunks without the work counter, and "moe_dyn_rounds" (0 = default) sets how many of the last

@@ -163,6 +163,10 @@ int mk36_set_option(const char* name, int value) {
         options().moe_batch = value ? 1 : 0;
         return MK36_OK;
     }
+    if (std::strcmp(name, "moe_wide") == 0) {
+        options().moe_wide = value > 0 ? value : 0;
+        return MK36_OK;
+    }
     if (std::strcmp(name, "moe_stages") == 0) {
         options().moe_stages = value > 0 ? value : 0;
         return MK36_OK;

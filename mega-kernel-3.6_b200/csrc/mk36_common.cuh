@@ -80,6 +80,7 @@ struct Options {
     int ring_mma = 0;       // 1: the MoE ring kernel contracts with mma.sync whatever the token count
     int moe_stream = 1;     // most tokens a call may have to run the stream kernel (0: never, 2: also two-token calls)
     int moe_batch = 1;      // 0: calls the stream kernel does not take use the ring kernel instead of the batch kernel
+    int moe_wide = 9;       // fewest tokens a call must have to run the wide kernel (0: never)
     int moe_stages = 0;     // > 0: ring depth of the MoE stream kernel (default: chosen from the shapes)
     int attn_stream = 1;    // 0: attention calls skip the streaming kernel (shared-memory ring) and use the register-staged one
     int dense_stream = 1;   // 0: one-token dense FFN calls use the tensor-core kernel instead of the streaming kernel
@@ -303,6 +304,13 @@ __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;
+}
+
+// 32 bytes at once (32-byte aligned): four lanes of a fragment load cover a whole 128-byte line of their row
+__device__ __forceinline__ void ld_stream_2u4(const void* p, uint4& a, uint4& b) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
 }
 
 template <typename T>

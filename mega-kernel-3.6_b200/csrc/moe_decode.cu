@@ -648,6 +648,8 @@ int moe_decode_ring_launch(const mk36_moe_args* a, const mk36_comm* comm, void* 
                            bool* handled);
 int moe_decode_stream_launch(const mk36_moe_args* a, const mk36_comm* comm, void* workspace, size_t workspace_bytes, cudaStream_t stream,
                              bool* handled);
+int moe_decode_wide_launch(const mk36_moe_args* a, const mk36_comm* comm, void* workspace, size_t workspace_bytes, cudaStream_t stream,
+                           bool* handled);
 int moe_decode_batch_launch(const mk36_moe_args* a, const mk36_comm* comm, void* workspace, size_t workspace_bytes, cudaStream_t stream,
                             bool* handled);
 
@@ -663,6 +665,13 @@ int moe_decode_launch(const mk36_moe_args* a, const mk36_comm* comm, void* works
         // faster of the two (34.9 against 40.1 us at the 35B shape)
         if (a->batch <= options().moe_stream && !options().ring_mma) {
             rc = moe_decode_stream_launch(a, comm, workspace, workspace_bytes, stream, &handled);
+            if (rc != MK36_OK || handled) return rc;
+        }
+        // nine tokens are where the batch kernel needs a second launch, which reads the experts that both halves chose
+        // twice (32 tokens at the 35B shape: 314 us as four launches, 204 as one); up to eight tokens the batch kernel's
+        // ring streams faster than the wide kernel's register loads
+        if (options().moe_wide > 0 && a->batch >= options().moe_wide && options().moe_batch && !options().ring_mma) {
+            rc = moe_decode_wide_launch(a, comm, workspace, workspace_bytes, stream, &handled);
             if (rc != MK36_OK || handled) return rc;
         }
         if (options().moe_batch && !options().ring_mma) {

@@ -572,7 +572,8 @@ def _kernel_schedule(graph: TaskGraph, wc: WorkerConfig, batch: int, context_len
             I, Is = cfg.moe_intermediate_size, cfg.shared_expert_intermediate_size
             distinct = min(batch * K, E)
             # one token: the stream kernel; more: the batch kernel, eight tokens per launch (the ring
-            # kernel, which takes as many tokens per launch as fit beside its activations, for shapes it refuses)
+            # kernel, which takes as many tokens per launch as fit beside its activations, for shapes it refuses);
+            # the schedule is by eights also where the launcher serves nine or more bf16 tokens with the wide kernel
             if batch <= KERNEL_GEOMETRY["moe_decode_stream_kernel"]["max_tokens"]:
                 kname, n_launches = "moe_decode_stream_kernel", 1
             elif moe_batch_kernel_fits(H, E, K, I, Is, sms):

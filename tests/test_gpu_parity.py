@@ -94,7 +94,7 @@ def test_moe_ring_kernel_tensor_core_consumers_match_oracle(name, cuda_device):
     assert_output_parity(got["out"], ref["out"], what=name + " (tensor-core consumers)")
 
 
-MOE_DEFAULT_OPTIONS = {"moe_stream": 1, "moe_batch": 1, "moe_static": 0, "moe_stages": 0, "moe_dyn_rounds": 0}
+MOE_DEFAULT_OPTIONS = {"moe_stream": 1, "moe_batch": 1, "moe_wide": 9, "moe_static": 0, "moe_stages": 0, "moe_dyn_rounds": 0}
 
 
 def _run_with_options(case, spec, device, options):
@@ -166,6 +166,28 @@ def test_moe_batch_kernel_ragged_and_shared_experts(shape, batch, dtype, same, c
     case = Case(f"moe_{shape}_b{batch}", "moe", lambda: None)
     spec = {"tensors": t, "top_k": shp.top_k}
     got = run_cuda(case, spec, cuda_device)
+    ref = run_oracle(case, spec)
+    assert_indices_exact(got["indices"], ref["indices"])
+    torch.testing.assert_close(got["weights"], ref["weights"], atol=1e-5, rtol=1e-4)
+    assert_output_parity(got["out"], ref["out"], what=case.name)
+    if same:
+        assert torch.equal(got["out"], got["out"][:1].expand_as(got["out"])), "identical tokens must give identical rows"
+
+
+@pytest.mark.parametrize("batch,same,fewest", [(1, False, 1), (8, False, 1), (9, True, 9), (17, False, 9), (32, False, 9), (32, True, 9), (33, False, 9)])
+def test_moe_wide_kernel_matches_oracle(batch, same, fewest, cuda_device):
+    """The kernel that takes up to 32 tokens per launch: one token, a full tile column, one more than that, more tokens
+    than two per warp, a full launch, 33 = 17 + 16, and identical tokens, whose experts need two and four entries."""
+    from golden_cases import Case
+    from mega_kernel_qwen36 import synthetic as syn
+
+    shp = syn.MOE_35B_A3B
+    t = syn.moe_tensors(shp, batch, 40 + batch, torch.bfloat16)
+    if same:
+        t["x"] = t["x"][:1].repeat(batch, 1).contiguous()
+    case = Case(f"moe_wide_b{batch}", "moe", lambda: None)
+    spec = {"tensors": t, "top_k": shp.top_k}
+    got = _run_with_options(case, spec, cuda_device, f"moe_stream=0,moe_wide={fewest}")
     ref = run_oracle(case, spec)
     assert_indices_exact(got["indices"], ref["indices"])
     torch.testing.assert_close(got["weights"], ref["weights"], atol=1e-5, rtol=1e-4)
