@@ -13,10 +13,17 @@
 // its chunks at kernel entry (the weights do not depend on x), and the consumers normalise x into
 // shared memory while the first chunks are in flight.  No grid barrier, so an ordinary launch.
 //
-//   chunk = as many whole rows as fit 32 KB (8 rows at an inner dimension of 2048); row r of chunk k
-//   is contracted by warp (k * rows + r) % 8 against one or two tokens; with more tokens a warp takes four
-//   rows and four tokens at a time (rows4_dot4);
-//   every consumer warp observes and releases every chunk (see moe_decode_stream.cu).
+//   One or two tokens: chunk = as many whole rows as fit 32 KB (8 rows at an inner dimension of 2048);
+//   row r of chunk k is contracted by warp (k * rows + r) % 8.  Inner dimensions that are not a multiple
+//   of 256 take three to eight tokens through the same chunks, four rows and four tokens at a time
+//   (rows4_dot4).
+//   Three to eight tokens: a CTA's rows are contiguous, cut into equal tiles of at most sixteen (one
+//   mma.sync.m16n8k16 tile, the tokens are its columns), and a stage is one tile by as many columns as
+//   fit 32 KB, brought in row by row with 16 bytes of padding.  Whole-row chunks filled 8 of the 16 rows
+//   at 2048 columns and 3 at 5120, met in shared memory after every chunk, and were read with bank
+//   conflicts: bound by shared memory instead of HBM.  Three tokens, the two projections of a 27B attention
+//   layer: 31 us less than with whole rows; LM head 2048 -> 248320, four tokens: 205 -> 197 us.
+//   Every consumer warp observes and releases every stage (see moe_decode_stream.cu).
 //
 // Arg-max: every warp keeps the best (value, row) of the rows it produced per token, on the rounded
 // output value with the lower row index winning ties (what arg-max over the stored output would
@@ -34,6 +41,8 @@ constexpr int kLinStageBytes = 32768;
 constexpr int kLinMaxStages = 6;
 constexpr int kLinMaxTokens = 8;
 constexpr int kLinMmaRows = 16;   // weight rows of one tensor-core tile
+constexpr int kLinPad = 8;        // tensor-core path, elements: rows in shared memory lie 16 bytes apart modulo 128, so that fragment loads meet all banks
+constexpr int kLinTileBytes = kLinMmaRows * (1024 + kLinPad) * 2;  // a stage of the tensor-core path
 constexpr int kLinMaxPieces = 8;  // 16-byte pieces of one token per consumer thread: inner dimension <= 16384
 
 struct LinearParams {
@@ -50,6 +59,8 @@ struct LinearParams {
     int nchunks;
     int nstages;
     int mma;      // 1: three to eight tokens on tensor-core instructions (tokens are the eight columns of the tile)
+    int kc;       // tensor-core path: columns of a stage, a multiple of 256 (rows: `rows`)
+    int stage_bytes;
     int off_red;  // tensor-core path: the warps' partial tiles, two buffers
     int lg_ppt;   // log2 of the 16-byte pieces of one token per consumer thread, rounded up to a power of two
     int off_x, off_ring, off_bars;
@@ -159,7 +170,12 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
     unsigned long long* empty_bar = full_bar + kLinMaxStages;
     const int R = p.nstages;
     const size_t rowK = (size_t)p.K;
-    const int my_chunks = (p.nchunks - cta + ncta - 1) / ncta;  // chunks cta, cta + ncta, ...
+    // plain path: chunks cta, cta + ncta, ...; tensor-core path: output rows [n0, n1) in tiles of p.rows, a tile in
+    // `ksteps` stages along the inner dimension
+    const int n0 = (int)(((long long)p.N * cta) / ncta), n1 = (int)(((long long)p.N * (cta + 1)) / ncta);
+    const int ksteps = p.mma ? (p.K + p.kc - 1) / p.kc : 1;
+    const int my_chunks = p.mma ? (n1 - n0 + p.rows - 1) / p.rows * ksteps : (p.nchunks - cta + ncta - 1) / ncta;
+    const size_t xstride = rowK + (p.mma ? kLinPad : 0);
 
     if (tid == 0 && cta == 0) trace_stamp(p.ctl, 0);
     if (tid < 2 * kLinMaxStages) mbar_init(&full_bar[tid], tid >= kLinMaxStages ? kLinConsumerWarps : 1);
@@ -175,9 +191,29 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
     // Producer warp: this CTA's chunks, in order, as stages come free
     // =====================================================================================
     if (is_producer) {
-        if (lane != 0) return;
         bool ok = true;
         int stage = 0, use = 0;
+        if (p.mma) {
+            int first = n0, kstep = 0;
+#pragma unroll 1
+            for (int k = 0; k < my_chunks; ++k) {
+                const int count = min(p.rows, n1 - first);
+                const int k0 = kstep * p.kc, width = min(p.kc, p.K - k0);
+                if (lane == 0) {
+                    if (use > 0) ok = mbar_wait(&empty_bar[stage], (unsigned)(use - 1) & 1u, &s_abort);
+                    if (ok) mbar_arrive_expect_tx(&full_bar[stage], (unsigned)(count * width * (int)sizeof(T)));
+                }
+                if (!__shfl_sync(kFullMask, ok ? 1 : 0, 0)) break;
+                if (lane < count)  // one row per lane
+                    bulk_copy_g2s(ring + (size_t)stage * p.stage_bytes + (size_t)lane * (p.kc + kLinPad) * sizeof(T),
+                                  static_cast<const T*>(p.w) + (size_t)(first + lane) * rowK + k0, (unsigned)(width * (int)sizeof(T)), &full_bar[stage]);
+                if (++kstep == ksteps) { kstep = 0; first += p.rows; }
+                if (++stage == R) { stage = 0; ++use; }
+            }
+            if (lane == 0 && !ok) atomicCAS(&p.ctl->status, 0, kStatusLinearProducer);
+            return;
+        }
+        if (lane != 0) return;
 #pragma unroll 1
         for (int k = 0; k < my_chunks && ok; ++k) {
             const int c = cta + k * ncta;
@@ -261,8 +297,8 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
             }
         }
         if (p.mma) {
-            for (int i = tid; i < (kLinMaxTokens - 1) * npieces; i += kLinConsumerThreads)
-                *reinterpret_cast<uint4*>(xs + rowK + 8 * (size_t)i) = make_uint4(0, 0, 0, 0);
+            for (int i = tid; i < (kLinMaxTokens - 1) * (int)(xstride >> 3); i += kLinConsumerThreads)
+                *reinterpret_cast<uint4*>(xs + xstride + 8 * (size_t)i) = make_uint4(0, 0, 0, 0);
         }
         if (tid == 0 && dirty != 0) s_dirty = 1;
         named_barrier(1, kLinConsumerThreads);
@@ -292,7 +328,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
                 for (int j = 0; j < kLinMaxPieces; ++j) {
                     const int b = first_tok + (j >> lg);
                     const int piece = tid + (j & (ppt - 1)) * kLinConsumerThreads;
-                    if (b < p.ntok && piece < npieces) *reinterpret_cast<uint4*>(xs + (size_t)b * rowK + 8 * piece) = xv[j];
+                    if (b < p.ntok && piece < npieces) *reinterpret_cast<uint4*>(xs + (size_t)b * xstride + 8 * piece) = xv[j];
                 }
                 continue;
             }
@@ -350,16 +386,16 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
                     T o[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) o[q] = from_float<T>(__fmul_rn(__fmul_rn(f[q], rs), g[q]));
-                    *reinterpret_cast<uint4*>(xs + (size_t)b * rowK + 8 * piece) = *reinterpret_cast<const uint4*>(o);
+                    *reinterpret_cast<uint4*>(xs + (size_t)b * xstride + 8 * piece) = *reinterpret_cast<const uint4*>(o);
                 }
             }
             // the next pass writes the other half of s_red; the one after it comes after this pass's barrier
         }
         if (p.mma) {
             // the tile has eight token columns: the ones beyond the batch are zero
-            const int npieces8 = (kLinMaxTokens - p.ntok) * (p.K >> 3);
+            const int npieces8 = (kLinMaxTokens - p.ntok) * (int)(xstride >> 3);
             for (int i = tid; i < npieces8; i += kLinConsumerThreads)
-                *reinterpret_cast<uint4*>(xs + (size_t)p.ntok * rowK + 8 * (size_t)i) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4*>(xs + (size_t)p.ntok * xstride + 8 * (size_t)i) = make_uint4(0, 0, 0, 0);
         }
         if (tid == 0 && dirty != 0) s_dirty = 1;
         named_barrier(1, kLinConsumerThreads);
@@ -373,6 +409,8 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
     const T* resid = static_cast<const T*>(p.residual);
     T* out = static_cast<T*>(p.out);
     unsigned long long best0 = 0ull, best1 = 0ull;  // lane l < 16: the best of tokens l % 4 and 4 + l % 4 among the rows this lane stored
+    float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};  // tensor-core path: this warp's share of the tile
+    int tile_first = n0, kstep = 0, buffer = 0;
     int stage = 0, use = 0, slot = 0;  // slot: (rows of the earlier chunks) % warps, the warp of the chunk's first row
 #pragma unroll 1
     for (int k = 0; k < my_chunks; ++k) {
@@ -385,38 +423,38 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
             if (++stage == R) { stage = 0; ++use; }
             continue;
         }
-        const int first = (cta + k * ncta) * p.rows;
-        const int count = min(p.rows, p.N - first);
-        const T* sbase = reinterpret_cast<const T*>(ring + (size_t)stage * kLinStageBytes);
+        const int first = p.mma ? tile_first : (cta + k * ncta) * p.rows;
+        const int count = min(p.rows, (p.mma ? n1 : p.N) - first);
+        const T* sbase = reinterpret_cast<const T*>(ring + (size_t)stage * p.stage_bytes);
         if (p.mma) {
-            // Tensor-core path: the chunk's rows (at most sixteen) are the rows of one m16n8k16 tile, the tokens its
-            // eight columns.  Warp w contracts the w-th eighth of the inner dimension for the whole tile: per 32-wide
-            // slice one 128-bit load per operand (rows g and g + 8 of the weights, token g of x; same permutation of
-            // the contraction index on both, see mk36_mma.cuh) and two MMAs.  The eight partial tiles meet in shared
-            // memory (two buffers, so one block-wide barrier per chunk), 128 threads finish one output each.
+            // Tensor-core path: a stage holds up to sixteen rows, the rows of one m16n8k16 tile, by p.kc columns; the
+            // tokens are the tile's eight columns.  Warp w contracts the w-th eighth of the stage for the whole tile: per
+            // 32-wide slice one 128-bit load per operand (rows g and g + 8 of the weights, token g of x; same permutation
+            // of the contraction index on both, see mk36_mma.cuh) and two MMAs.  The accumulators stay in the warp until
+            // the tile's last stage; then the eight partial tiles meet in shared memory (two buffers, so one block-wide
+            // barrier per tile) and 128 threads finish one output each.
             const int g = lane >> 2, t = lane & 3;
-            const int nsl = p.K >> 8;  // 32-wide slices per warp
-            float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
-            const T* alo = sbase + (size_t)g * rowK + 8 * t;
-            const T* ahi = sbase + (size_t)(g + 8) * rowK + 8 * t;
-            const T* bx = xs + (size_t)g * rowK + 8 * t;
-            const bool lo_live = g < count, hi_live = g + 8 < count;
-            const uint4 zero = make_uint4(0, 0, 0, 0);
+            const int k0 = kstep * p.kc;
+            const int nsl = min(p.kc, p.K - k0) >> 8;  // 32-wide slices per warp
+            const int kw = warp * nsl * 32 + 8 * t;
+            const T* alo = sbase + (size_t)min(g, count - 1) * (p.kc + kLinPad) + kw;  // rows beyond the tile repeat its last one: not stored
+            const T* ahi = sbase + (size_t)min(g + 8, count - 1) * (p.kc + kLinPad) + kw;
+            const T* bx = xs + (size_t)g * xstride + k0 + kw;
 #pragma unroll 4
-            for (int sl = 0; sl < nsl; ++sl) {
-                const int kb = (warp * nsl + sl) * 32;
-                const uint4 a0 = lo_live ? lds128(alo + kb) : zero;
-                const uint4 a1 = hi_live ? lds128(ahi + kb) : zero;
-                const uint4 bb = lds128(bx + kb);
-                mma_slice32<T>(d0, d1, a0, a1, bb);
-            }
-            float* red = reinterpret_cast<float*>(smem + p.off_red) + (size_t)(k & 1) * (kLinConsumerWarps * kLinMmaRows * 8);
-            float* mine = red + (size_t)warp * (kLinMmaRows * 8);
-            *reinterpret_cast<float2*>(mine + g * 8 + 2 * t) = make_float2(d0[0] + d1[0], d0[1] + d1[1]);
-            *reinterpret_cast<float2*>(mine + (g + 8) * 8 + 2 * t) = make_float2(d0[2] + d1[2], d0[3] + d1[3]);
+            for (int sl = 0; sl < nsl; ++sl) mma_slice32<T>(d0, d1, lds128(alo + 32 * sl), lds128(ahi + 32 * sl), lds128(bx + 32 * sl));
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_bar[stage]);  // the weights of this stage have been read
             if (++stage == R) { stage = 0; ++use; }
+            if (++kstep < ksteps) continue;
+            float* red = reinterpret_cast<float*>(smem + p.off_red) + (size_t)buffer * (kLinConsumerWarps * kLinMmaRows * 8);
+            float* mine = red + (size_t)warp * (kLinMmaRows * 8);
+            *reinterpret_cast<float2*>(mine + g * 8 + 2 * t) = make_float2(d0[0] + d1[0], d0[1] + d1[1]);
+            *reinterpret_cast<float2*>(mine + (g + 8) * 8 + 2 * t) = make_float2(d0[2] + d1[2], d0[3] + d1[3]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { d0[i] = 0.0f; d1[i] = 0.0f; }
+            kstep = 0;
+            tile_first += p.rows;
+            buffer ^= 1;
             named_barrier(1, kLinConsumerThreads);
             if (tid < kLinMmaRows * 8) {
                 const int row = tid >> 3, tok = tid & 7;
@@ -596,8 +634,20 @@ int mk36_linear_decode(const mk36_linear_args* a, void* workspace, size_t worksp
     // three to eight tokens: tensor-core tiles when the inner dimension splits into 32-wide slices over the eight warps
     p.mma = (options().linear_mma > 0 && a->batch >= options().linear_mma && K % 256 == 0) ? 1 : 0;
     p.rows = kLinStageBytes / (K * 2);
-    if (p.mma && p.rows > kLinMmaRows) p.rows = kLinMmaRows;
     p.nchunks = (N + p.rows - 1) / p.rows;
+    p.kc = 0;
+    p.stage_bytes = kLinStageBytes;
+    int grid = p.nchunks < dev->sm_count ? p.nchunks : dev->sm_count;
+    if (p.mma) {
+        // a CTA's rows are contiguous and cut into equal tiles of at most sixteen; a stage is as many columns of a tile
+        // as fit, so that it holds about 32 KB whatever the inner dimension
+        grid = N < dev->sm_count ? N : dev->sm_count;
+        const int per_cta = (N + grid - 1) / grid, tiles = (per_cta + kLinMmaRows - 1) / kLinMmaRows;
+        p.rows = (per_cta + tiles - 1) / tiles;
+        p.kc = (kLinTileBytes / 2 / p.rows - kLinPad) / 256 * 256;
+        if (p.kc > K) p.kc = K;
+        p.stage_bytes = kLinTileBytes;
+    }
     {
         const int ppt = (K / 8 + kLinConsumerThreads - 1) / kLinConsumerThreads;
         p.lg_ppt = 0;
@@ -613,15 +663,14 @@ int mk36_linear_decode(const mk36_linear_args* a, void* workspace, size_t worksp
     p.off_bars = take(2 * kLinMaxStages * 8, 16);
     const int xtok = p.mma ? kLinMaxTokens : (a->batch > 2 ? (a->batch + 3) / 4 * 4 : a->batch);  // groups of three tokens read a fourth vector
     p.off_red = take(p.mma ? (size_t)2 * kLinConsumerWarps * kLinMmaRows * 8 * 4 : 0, 16);
-    p.off_x = take((size_t)xtok * K * 2, 128);
+    p.off_x = take((size_t)xtok * (K + (p.mma ? kLinPad : 0)) * 2, 128);
     p.off_ring = take(0, 128);
     const long long room = (long long)dev->max_smem_optin - (long long)off - 1024;
-    int nstages = (int)(room / kLinStageBytes);
+    int nstages = (int)(room / p.stage_bytes);
     if (nstages > kLinMaxStages) nstages = kLinMaxStages;
     if (nstages < 2) MK36_FAIL(MK36_ERR_UNSUPPORTED, "linear_decode: shapes do not fit in shared memory");
     p.nstages = nstages;
-    const size_t smem_bytes = (size_t)p.off_ring + (size_t)nstages * kLinStageBytes;
-    const int grid = p.nchunks < dev->sm_count ? p.nchunks : dev->sm_count;
+    const size_t smem_bytes = (size_t)p.off_ring + (size_t)nstages * p.stage_bytes;
 
     const void* kernel = (a->dtype == MK36_BF16) ? (const void*)linear_decode_kernel<__nv_bfloat16> : (const void*)linear_decode_kernel<__half>;
     {
