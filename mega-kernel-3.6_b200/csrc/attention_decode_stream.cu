@@ -393,7 +393,10 @@ __global__ void __launch_bounds__(kAsThreads, 1) attention_decode_stream_kernel(
     named_barrier(1, kAsConsumerThreads);
     if (tracer) trace_stamp(p.ctl, 7);
     if (!s_flag) return;
-    attention_merge_items<T>(p, blockIdx.x * kAsConsumerWarps + warp, gridDim.x * kAsConsumerWarps, lane);
+    // lanes on the splits when there are many (one or two batch items), on the channels when there are few
+    const int item0 = warp * gridDim.x + blockIdx.x;  // neighbouring items on different SMs
+    if (D % 128 == 0 && p.splits <= kAttnMergeFewSplits) attention_merge_few_splits<T>(p, item0, gridDim.x * kAsConsumerWarps, lane);
+    else attention_merge_items<T>(p, blockIdx.x * kAsConsumerWarps + warp, gridDim.x * kAsConsumerWarps, lane);
     if (tracer) trace_stamp(p.ctl, 6);
 }
 
