@@ -96,7 +96,8 @@ MK36_API int mk36_workspace_status(void* workspace, void* stream, int* device_st
  * chunks without the work counter, and "moe_dyn_rounds" (0 = default) sets how many of the last
  * rounds of gate/up chunks go through that counter; these exist for measurements.  One-token dense FFN calls normally
  * run the streaming kernel; "dense_stream" = 0 sends them to the tensor-core kernel that serves the
- * larger batches.  Attention calls with bf16 / f16 caches normally run the streaming kernel (cache
+ * larger batches, which is fed by a shared-memory ring unless "dense_tiles" = 0 or the shape leaves too little room
+ * for one.  Attention calls with bf16 / f16 caches normally run the streaming kernel (cache
  * chunks of all KV heads through a shared-memory ring); "attn_stream" = 0 sends them to the
  * tensor-core kernel that stages the cache in registers.  "linear_mma" is the smallest token count
  * for which a projection (mk36_linear_decode) runs on tensor-core tiles (default 3, 0 = never).  Unknown names return

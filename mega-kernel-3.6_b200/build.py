@@ -37,6 +37,7 @@ CUDA_SOURCES = [
     "moe_decode_wide.cu",
     "dense_ffn_decode.cu",
     "dense_ffn_mma.cu",
+    "dense_ffn_tiles.cu",
     "dense_ffn_stream.cu",
     "attention_append.cu",
     "attention_decode.cu",

@@ -8,6 +8,8 @@
 
 namespace mk36 {
 int moe_decode_launch(const mk36_moe_args* a, const mk36_comm* comm, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+int dense_ffn_tiles_launch(const mk36_dense_ffn_args* a, const mk36_comm* comm, void* workspace, size_t workspace_bytes, cudaStream_t stream,
+                           bool* handled);
 int dense_ffn_mma_launch(const mk36_dense_ffn_args* a, const mk36_comm* comm, void* workspace, size_t workspace_bytes, cudaStream_t stream,
                          bool* handled);
 int dense_ffn_stream_launch(const mk36_dense_ffn_args* a, const mk36_comm* comm, void* workspace, size_t workspace_bytes, cudaStream_t stream,
@@ -50,6 +52,12 @@ int dense_launch(const mk36_dense_ffn_args* a, const mk36_moe_args* m, const mk3
         bool handled = false;
         if (options().dense_stream) {
             const int rc = dense_ffn_stream_launch(a, comm, workspace, workspace_bytes, stream, &handled);
+            if (rc != MK36_OK || handled) return rc;
+        }
+        // the ring needs room for three stages beside the eight tokens (hidden size up to about 7000) and a tile per CTA;
+        // 27B shape, eight tokens: 134 us with register loads, 114 through the ring
+        if (options().dense_tiles) {
+            const int rc = dense_ffn_tiles_launch(a, comm, workspace, workspace_bytes, stream, &handled);
             if (rc != MK36_OK || handled) return rc;
         }
         const int rc = dense_ffn_mma_launch(a, comm, workspace, workspace_bytes, stream, &handled);

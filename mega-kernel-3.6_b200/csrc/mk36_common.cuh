@@ -84,6 +84,7 @@ struct Options {
     int moe_stages = 0;     // > 0: ring depth of the MoE stream kernel (default: chosen from the shapes)
     int attn_stream = 1;    // 0: attention calls skip the streaming kernel (shared-memory ring) and use the register-staged one
     int dense_stream = 1;   // 0: one-token dense FFN calls use the tensor-core kernel instead of the streaming kernel
+    int dense_tiles = 1;    // 0: dense FFN calls of several tokens use the register-staged tensor-core kernel instead of the ring-fed one
     int moe_dyn_rounds = 0; // > 0: rounds of gate/up chunks at the end of the stream dealt through the work counter (default: 4 in the stream kernel, 2 in the batch kernel)
     int linear_mma = 3;     // fewest tokens for which a projection runs on tensor-core tiles (0: never)
     int moe_static = 0;     // 1: the MoE stream kernel deals its gate/up chunks statically (no work counter)

@@ -453,6 +453,7 @@ KERNEL_GEOMETRY = {
     "moe_decode_batch_kernel": {"block": 416, "grid_barriers": 1, "max_tokens": 8},
     "moe_decode_ring_kernel": {"block": 416, "grid_barriers": 2, "max_tokens": 8},
     "dense_ffn_mma_kernel": {"block": 512, "grid_barriers": 1, "max_tokens": 8},
+    "dense_ffn_tiles_kernel": {"block": 288, "grid_barriers": 1, "max_tokens": 8},
     "attention_decode_stream_kernel": {"block": 288, "grid_barriers": 1},
     "dense_ffn_stream_kernel": {"block": 416, "grid_barriers": 1, "max_tokens": 1},
     "linear_attention_kernel": {"block": 256, "grid_barriers": 0},  # unaligned shapes only
@@ -596,7 +597,9 @@ def _kernel_schedule(graph: TaskGraph, wc: WorkerConfig, batch: int, context_len
         elif task.kind == "dense_down":
             group = by_layer.pop(li, []) + [task]
             I = cfg.intermediate_size
-            dense_kernel = "dense_ffn_stream_kernel" if batch == 1 else "dense_ffn_mma_kernel"  # one token streams, more use the tensor cores
+            # one token streams; more use the tensor cores, fed by a ring where three stages fit beside the tokens
+            ring_fits = _SMEM_OPTIN - 1024 - 128 - 8192 - 16 * (H + 8) >= 3 * 33024 and min(H, I) >= sms
+            dense_kernel = "dense_ffn_stream_kernel" if batch == 1 else "dense_ffn_tiles_kernel" if ring_fits else "dense_ffn_mma_kernel"
             launches.append(KernelLaunch(
                 name=f"layer_{li}_dense_ffn", entry_point="mk36_dense_ffn_decode", task_ids=tuple(t.id for t in group),
                 kernel=dense_kernel, launches=_ceil_div(batch, KERNEL_GEOMETRY[dense_kernel]["max_tokens"]),

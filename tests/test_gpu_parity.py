@@ -243,6 +243,32 @@ def test_dense_one_token_through_the_tensor_core_kernel(name, cuda_device):
     assert_output_parity(got["out"], run_oracle(case, spec)["out"], what=name + " (tensor-core kernel)")
 
 
+@pytest.mark.parametrize("batch,hidden,intermediate,dtype,tiles", [
+    (2, 160, 160, torch.bfloat16, 1),      # one or two rows and channels per CTA, stages narrower than a warp round
+    (3, 1184, 1184, torch.float16, 1),     # eight of each per CTA: a whole gate/up tile, half a down tile
+    (5, 2400, 1216, torch.bfloat16, 1),    # seventeen rows: two down tiles; column remainders in both phases
+    (8, 5120, 2176, torch.bfloat16, 1),    # a tensor-parallel slice
+    (9, 5120, 2176, torch.float16, 1),     # a second launch of one token
+    (8, 5120, 17408, torch.bfloat16, 1),   # the whole layer
+    (8, 5120, 2176, torch.bfloat16, 0),    # the register-staged kernel, which shapes without room for the ring take
+], ids=lambda v: str(v).replace("torch.", ""))
+def test_dense_tensor_core_tiles_match_oracle(batch, hidden, intermediate, dtype, tiles, cuda_device):
+    """The ring-fed tensor-core kernel at the edges of its tiles and stages."""
+    from golden_cases import Case
+    from mega_kernel_qwen36 import cabi
+    from mega_kernel_qwen36 import synthetic as syn
+
+    spec = {"tensors": syn.dense_tensors(syn.DenseShape(hidden, intermediate), batch, 70 + batch, dtype)}
+    case = Case(f"dense_{hidden}_{intermediate}_b{batch}", "dense", lambda: None)
+    lib = cabi.load()
+    cabi.check(lib.mk36_set_option(b"dense_tiles", tiles))
+    try:
+        got = run_cuda(case, spec, cuda_device)
+    finally:
+        cabi.check(lib.mk36_set_option(b"dense_tiles", 1))
+    assert_output_parity(got["out"], run_oracle(case, spec)["out"], what=case.name)
+
+
 @pytest.mark.parametrize("name", ["attn_27b_bf16_t1000", "attn_35b_bf16_t4096", "attn_35b_bf16_b2_t2500"])
 def test_attention_general_kernel_matches_oracle(name, cuda_device):
     """Shapes that normally take the tensor-core attention kernel, forced through the general one."""
