@@ -375,20 +375,22 @@ __global__ void __launch_bounds__(kMoeThreads, 1) moe_decode_kernel(const MoePar
     for (int idx = tid; idx < npairs * a_stride; idx += kMoeThreads) acts[idx] = 0.0f;
     for (int idx = tid; idx < p.ntok * sa_stride; idx += kMoeThreads) sacts[idx] = 0.0f;
     __syncthreads();
-    for (int u = 0; u < n_unique; ++u) {
-        unsigned long long m = s_uniq_m[u];
-        while (m) {
-            const int pair = __ffsll((long long)m) - 1;
-            m &= m - 1;
+    // all pairs' channels in one loop, several in flight per thread: pair after pair, each was a round trip to L2 (small
+    // example, f32, eight tokens: 57 us that way, 40 this way; one token 18.8 and 18.0)
+#pragma unroll 4
+    for (int idx = tid; idx < npairs * p.I; idx += kMoeThreads) {
+        const int pair = idx / p.I, i = idx - pair * p.I;
+        const int e = s_pair_e[pair] - p.expert_base;
+        if (e >= 0 && e < p.local_experts) {
             const float* g = p.gu + (size_t)pair * 2 * p.I;
-            for (int i = tid; i < p.I; i += kMoeThreads)
-                acts[pair * a_stride + split_index(i, a_half)] = silu(__ldcg(g + i)) * __ldcg(g + p.I + i);
+            acts[pair * a_stride + split_index(i, a_half)] = silu(__ldcg(g + i)) * __ldcg(g + p.I + i);
         }
     }
-    for (int b = 0; b < p.ntok; ++b) {
+#pragma unroll 4
+    for (int idx = tid; idx < p.ntok * p.Is; idx += kMoeThreads) {
+        const int b = idx / p.Is, i = idx - b * p.Is;
         const float* g = p.sgu + (size_t)b * 2 * p.Is;
-        for (int i = tid; i < p.Is; i += kMoeThreads)
-            sacts[b * sa_stride + split_index(i, sa_half)] = silu(__ldcg(g + i)) * __ldcg(g + p.Is + i);
+        sacts[b * sa_stride + split_index(i, sa_half)] = silu(__ldcg(g + i)) * __ldcg(g + p.Is + i);
     }
     __syncthreads();
     if (tracer) trace_stamp(p.ctl, 8);
