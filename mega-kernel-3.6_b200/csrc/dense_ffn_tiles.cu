@@ -133,7 +133,13 @@ __global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const De
                 issue(row, count, min(p.kcc, p.I - k * p.kcc), p.kcc);
             }
         }
-        if (!ok && lane == 0) atomicCAS(&p.ctl->status, 0, kStatusMoeRingProducer);
+        if (lane == 0) {
+            if (!ok) {
+                atomicCAS(&p.ctl->status, 0, kStatusMoeRingProducer);
+                if (--stage < 0) { stage = R - 1; --use; }  // the stage that was not filled
+            }
+            ring_drain(full_bar, R, stage, use);
+        }
         return;
     }
 
@@ -205,7 +211,7 @@ __global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const De
     T* act_lo = static_cast<T*>(p.act_lo);
     int buffer = 0;
 #pragma unroll 1
-    for (int first = c0; first < c1 && ok; first += p.pa) {
+    for (int first = c0; first < c1; first += p.pa) {
         const int count = min(p.pa, c1 - first);
         const int rl = min(g, count - 1);  // rows beyond the tile repeat its last one: not stored
         float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
@@ -222,8 +228,9 @@ __global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const De
             for (int c = 32 * warp; c < width; c += 32 * kDtWarps) mma_slice32<T>(d0, d1, lds128(alo + c), lds128(ahi + c), lds128(bx + c));
             release();
         }
-        if (!ok) break;
-        // the warps' shares of the tile meet; two buffers, so one barrier per tile
+        // The warps' shares of the tile meet; two buffers, so one barrier per tile.  A warp whose wait has run out comes to
+        // every tile's barrier like the others: the barrier has no limit, and they may be some tiles from giving up.  What
+        // such a CTA stores stays in the scratch buffer, because it does not arrive at the grid barrier.
         float* red = reinterpret_cast<float*>(smem + p.off_red) + buffer * (kDtWarps * 128);
         float* mine = red + warp * 128;
         *reinterpret_cast<float2*>(mine + g * 8 + 2 * t) = make_float2(d0[0] + d1[0], d0[1] + d1[1]);
@@ -246,13 +253,13 @@ __global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const De
         }
         buffer ^= 1;
     }
-    if (!ok) atomicCAS(&p.ctl->status, 0, kStatusMoeRingConsumer);
+    if (*(volatile int*)&s_abort != 0) atomicCAS(&p.ctl->status, 0, kStatusMoeRingConsumer);
     if (tracer) trace_stamp(p.ctl, 2);
 
     // ---- grid barrier: all activations are in the workspace ----
     named_barrier(1, kDtConsumers);
     if (tid == 0) {
-        bool fine = ok && (*(volatile int*)&s_abort == 0);
+        bool fine = (*(volatile int*)&s_abort == 0);  // set before the barrier by a warp whose wait has run out
         if (fine) {
             fine = barrier_wait(p.ctl, barrier_arrive(p.ctl, ncta, 0), kStatusDenseBarrier);
             if (fine) barrier_finish(p.ctl, ncta);

@@ -96,6 +96,19 @@ __device__ __forceinline__ void named_barrier(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The last thing a producer lane does, with (stage, use) the next place it would have filled: waits, with a limit for each
+// stage, until the copies that it has armed have landed.  Consumers that gave up leave without looking at them, and a CTA
+// must not end with a copy into its shared memory on the way.  (Without a failure the consumers wait for the same copies.)
+static __device__ __noinline__ void ring_drain(unsigned long long* full_bar, int depth, int stage, int use) {
+    for (int s = 0; s < depth; ++s) {
+        const int last = (s < stage) ? use : use - 1;  // the last use of this stage, if any
+        if (last < 0) continue;
+        const unsigned long long t0 = global_timer_ns();
+        while (!mbar_try_wait(&full_bar[s], (unsigned)last & 1u) && global_timer_ns() - t0 <= kWaitLimitNs) {
+        }
+    }
+}
+
 __device__ __forceinline__ uint4 lds128(const void* p) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_addr(p)));

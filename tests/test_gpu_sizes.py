@@ -64,3 +64,53 @@ def test_attention_block_reads_caches_longer_than_the_context(heads, position, c
     assert_output_parity(dev["v_cache"][:, position].cpu(), v_ref[:, position], what="block value")
     rest = [i for i in range(capacity) if i != position]
     assert torch.equal(dev["k_cache"][:, rest].cpu(), cache["k_cache"][:, rest]) and torch.equal(dev["v_cache"][:, rest].cpu(), cache["v_cache"][:, rest])
+
+
+@pytest.mark.parametrize("kernel", ["dense_tiles"])
+def test_ring_fed_kernels_leave_together_when_their_waits_fail(kernel, cuda_device):
+    """Behind a wait that has given up (made on the host side: a barrier that expects an arrival nobody makes) the status is
+    still reported and nothing is stored; with the workspace initialised again the same call gives the operator's result."""
+    import ctypes
+
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import cabi, synthetic as syn
+
+    lib, dev = cabi.load(), cuda_device
+    nbytes = lib.mk36_workspace_bytes()
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    stream = torch.cuda.current_stream().cuda_stream
+    status = ctypes.c_int(-1)
+    best = expect_best = None
+    if kernel == "dense_tiles":
+        t = {k: v.to(dev) for k, v in syn.dense_tensors(syn.DenseShape(2400, 1216), 5, seed=5).items()}
+        out = torch.empty_like(t["x"])
+        args = cabi.DenseFfnArgs(x=t["x"].data_ptr(), norm_weight=t["norm_weight"].data_ptr(), gate_weight=t["gate_weight"].data_ptr(),
+                                 up_weight=t["up_weight"].data_ptr(), down_weight=t["down_weight"].data_ptr(), out=out.data_ptr(),
+                                 partial_out=None, dtype=cabi.MK36_BF16, batch=5, hidden=2400, intermediate=1216, add_residual=1, eps=1e-6)
+        call = lambda: lib.mk36_dense_ffn_decode(args, ws.data_ptr(), nbytes, stream)
+        expect = mk.dense_ffn_decode(t["x"], mk.DenseFfnWeights(*[t[f] for f in syn.DENSE_WEIGHT_FIELDS]))
+    else:  # 2304 = a whole stage of columns and a narrower one
+        batch, argmax = (2 if "rows" in kernel else 4), "argmax" in kernel
+        t = {k: v.to(dev) for k, v in syn.projection_tensors(2304, 5000, batch, seed=9, norm=True, residual=True).items()}
+        out = torch.empty(batch, 5000, dtype=torch.bfloat16, device=dev)
+        best = torch.empty(batch, dtype=torch.int64, device=dev) if argmax else None
+        args = cabi.LinearArgs(x=t["x"].data_ptr(), norm_weight=t["norm_weight"].data_ptr(), weight=t["weight"].data_ptr(),
+                               residual=t["residual"].data_ptr(), out=out.data_ptr(), argmax=best.data_ptr() if argmax else None,
+                               dtype=cabi.MK36_BF16, batch=batch, in_features=2304, out_features=5000, eps=1e-6)
+        call = lambda: lib.mk36_linear_decode(args, ws.data_ptr(), nbytes, stream)
+        expect, expect_best = mk.linear_decode(t["x"], t["weight"], norm_weight=t["norm_weight"], residual=t["residual"], return_argmax=True)
+    for spoilt in (True, False):
+        cabi.check(lib.mk36_workspace_init(ws.data_ptr(), nbytes, stream))
+        out.fill_(5.0)
+        if best is not None:
+            best.fill_(-7)
+        if spoilt:
+            cabi.check(lib.mk36_selftest_bounded_wait(ws.data_ptr(), nbytes, stream, 20))
+        cabi.check(call())
+        rc = lib.mk36_workspace_status(ws.data_ptr(), stream, ctypes.byref(status))
+        if spoilt:
+            assert rc == cabi.MK36_ERR_BARRIER_TIMEOUT and status.value == 901
+            assert bool((out == 5.0).all()) and (best is None or bool((best == -7).all()))
+        else:
+            assert rc == 0 and status.value == 0
+            assert torch.equal(out, expect) and (best is None or torch.equal(best, expect_best))
