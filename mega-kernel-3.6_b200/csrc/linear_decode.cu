@@ -58,9 +58,7 @@ struct LinearParams {
     int rows;     // weight rows per chunk
     int nchunks;
     int nstages;
-    int mma;      // 1: three to eight tokens on tensor-core instructions (tokens are the eight columns of the tile)
     int kc;       // tensor-core path: columns of a stage, a multiple of 256 (rows: `rows`)
-    int stage_bytes;
     int off_red;  // tensor-core path: the warps' partial tiles, two buffers
     int lg_ppt;   // log2 of the 16-byte pieces of one token per consumer thread, rounded up to a power of two
     int off_x, off_ring, off_bars;
@@ -149,7 +147,10 @@ __device__ __forceinline__ unsigned long long argmax_key(float v, int row) {
     return ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (unsigned)row);
 }
 
-template <typename T>
+// MMA: three to eight tokens on tensor-core instructions (tokens are the eight columns of the tile).  A kernel of its own:
+// decided at run time inside one kernel, the same choice cost the calls of one and two tokens 1 to 7 % (35B q|k|v
+// projection, two tokens: 14.5 us that way, 12.4 this way; LM head, one token: 198.7 and 191.3).
+template <typename T, bool MMA>
 __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const LinearParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_abort;
@@ -168,14 +169,15 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
     unsigned char* ring = smem + p.off_ring;
     unsigned long long* full_bar = reinterpret_cast<unsigned long long*>(smem + p.off_bars);
     unsigned long long* empty_bar = full_bar + kLinMaxStages;
+    constexpr int kStageBytes = MMA ? kLinTileBytes : kLinStageBytes;
     const int R = p.nstages;
     const size_t rowK = (size_t)p.K;
     // plain path: chunks cta, cta + ncta, ...; tensor-core path: output rows [n0, n1) in tiles of p.rows, a tile in
     // `ksteps` stages along the inner dimension
     const int n0 = (int)(((long long)p.N * cta) / ncta), n1 = (int)(((long long)p.N * (cta + 1)) / ncta);
-    const int ksteps = p.mma ? (p.K + p.kc - 1) / p.kc : 1;
-    const int my_chunks = p.mma ? (n1 - n0 + p.rows - 1) / p.rows * ksteps : (p.nchunks - cta + ncta - 1) / ncta;
-    const size_t xstride = rowK + (p.mma ? kLinPad : 0);
+    const int ksteps = MMA ? (p.K + p.kc - 1) / p.kc : 1;
+    const int my_chunks = MMA ? (n1 - n0 + p.rows - 1) / p.rows * ksteps : (p.nchunks - cta + ncta - 1) / ncta;
+    const size_t xstride = rowK + (MMA ? kLinPad : 0);
 
     if (tid == 0 && cta == 0) trace_stamp(p.ctl, 0);
     if (tid < 2 * kLinMaxStages) mbar_init(&full_bar[tid], tid >= kLinMaxStages ? kLinConsumerWarps : 1);
@@ -193,7 +195,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
     if (is_producer) {
         bool ok = true;
         int stage = 0, use = 0;
-        if (p.mma) {
+        if (MMA) {
             int first = n0, kstep = 0;
 #pragma unroll 1
             for (int k = 0; k < my_chunks; ++k) {
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
                 }
                 if (!__shfl_sync(kFullMask, ok ? 1 : 0, 0)) break;
                 if (lane < count)  // one row per lane
-                    bulk_copy_g2s(ring + (size_t)stage * p.stage_bytes + (size_t)lane * (p.kc + kLinPad) * sizeof(T),
+                    bulk_copy_g2s(ring + (size_t)stage * kStageBytes + (size_t)lane * (p.kc + kLinPad) * sizeof(T),
                                   static_cast<const T*>(p.w) + (size_t)(first + lane) * rowK + k0, (unsigned)(width * (int)sizeof(T)), &full_bar[stage]);
                 if (++kstep == ksteps) { kstep = 0; first += p.rows; }
                 if (++stage == R) { stage = 0; ++use; }
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
                 }
             }
         }
-        if (p.mma) {
+        if (MMA) {
             for (int i = tid; i < (kLinMaxTokens - 1) * (int)(xstride >> 3); i += kLinConsumerThreads)
                 *reinterpret_cast<uint4*>(xs + xstride + 8 * (size_t)i) = make_uint4(0, 0, 0, 0);
         }
@@ -391,7 +393,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
             }
             // the next pass writes the other half of s_red; the one after it comes after this pass's barrier
         }
-        if (p.mma) {
+        if (MMA) {
             // the tile has eight token columns: the ones beyond the batch are zero
             const int npieces8 = (kLinMaxTokens - p.ntok) * (int)(xstride >> 3);
             for (int i = tid; i < npieces8; i += kLinConsumerThreads)
@@ -423,10 +425,10 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
             if (++stage == R) { stage = 0; ++use; }
             continue;
         }
-        const int first = p.mma ? tile_first : (cta + k * ncta) * p.rows;
-        const int count = min(p.rows, (p.mma ? n1 : p.N) - first);
-        const T* sbase = reinterpret_cast<const T*>(ring + (size_t)stage * p.stage_bytes);
-        if (p.mma) {
+        const int first = MMA ? tile_first : (cta + k * ncta) * p.rows;
+        const int count = min(p.rows, (MMA ? n1 : p.N) - first);
+        const T* sbase = reinterpret_cast<const T*>(ring + (size_t)stage * kStageBytes);
+        if (MMA) {
             // Tensor-core path: a stage holds up to sixteen rows, the rows of one m16n8k16 tile, by p.kc columns; the
             // tokens are the tile's eight columns.  Warp w contracts the w-th eighth of the stage for the whole tile: per
             // 32-wide slice one 128-bit load per operand (rows g and g + 8 of the weights, token g of x; same permutation
@@ -557,7 +559,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
     if (tid == 0 && cta == ncta - 1) trace_stamp(p.ctl, 3);
 
     // ---- arg-max: CTA-wide maxima first ----
-    if (p.argmax && p.mma) {
+    if (p.argmax && MMA) {
         if (tid < kLinMmaRows * 8 && best0 != 0ull) atomicMax(&s_best[tid & 7], best0);
     } else if (p.argmax && lane < 16) {
         if (best0 != 0ull) atomicMax(&s_best[lane & 3], best0);
@@ -632,13 +634,13 @@ int mk36_linear_decode(const mk36_linear_args* a, void* workspace, size_t worksp
     p.N = N;
     p.eps = a->eps;
     // three to eight tokens: tensor-core tiles when the inner dimension splits into 32-wide slices over the eight warps
-    p.mma = (options().linear_mma > 0 && a->batch >= options().linear_mma && K % 256 == 0) ? 1 : 0;
+    const bool mma = options().linear_mma > 0 && a->batch >= options().linear_mma && K % 256 == 0;
     p.rows = kLinStageBytes / (K * 2);
     p.nchunks = (N + p.rows - 1) / p.rows;
     p.kc = 0;
-    p.stage_bytes = kLinStageBytes;
+    const int stage_bytes = mma ? kLinTileBytes : kLinStageBytes;
     int grid = p.nchunks < dev->sm_count ? p.nchunks : dev->sm_count;
-    if (p.mma) {
+    if (mma) {
         // a CTA's rows are contiguous and cut into equal tiles of at most sixteen; a stage is as many columns of a tile
         // as fit, so that it holds about 32 KB whatever the inner dimension
         grid = N < dev->sm_count ? N : dev->sm_count;
@@ -646,7 +648,6 @@ int mk36_linear_decode(const mk36_linear_args* a, void* workspace, size_t worksp
         p.rows = (per_cta + tiles - 1) / tiles;
         p.kc = (kLinTileBytes / 2 / p.rows - kLinPad) / 256 * 256;
         if (p.kc > K) p.kc = K;
-        p.stage_bytes = kLinTileBytes;
     }
     {
         const int ppt = (K / 8 + kLinConsumerThreads - 1) / kLinConsumerThreads;
@@ -661,18 +662,20 @@ int mk36_linear_decode(const mk36_linear_args* a, void* workspace, size_t worksp
         return (int)at;
     };
     p.off_bars = take(2 * kLinMaxStages * 8, 16);
-    const int xtok = p.mma ? kLinMaxTokens : (a->batch > 2 ? (a->batch + 3) / 4 * 4 : a->batch);  // groups of three tokens read a fourth vector
-    p.off_red = take(p.mma ? (size_t)2 * kLinConsumerWarps * kLinMmaRows * 8 * 4 : 0, 16);
-    p.off_x = take((size_t)xtok * (K + (p.mma ? kLinPad : 0)) * 2, 128);
+    const int xtok = mma ? kLinMaxTokens : (a->batch > 2 ? (a->batch + 3) / 4 * 4 : a->batch);  // groups of three tokens read a fourth vector
+    p.off_red = take(mma ? (size_t)2 * kLinConsumerWarps * kLinMmaRows * 8 * 4 : 0, 16);
+    p.off_x = take((size_t)xtok * (K + (mma ? kLinPad : 0)) * 2, 128);
     p.off_ring = take(0, 128);
     const long long room = (long long)dev->max_smem_optin - (long long)off - 1024;
-    int nstages = (int)(room / p.stage_bytes);
+    int nstages = (int)(room / stage_bytes);
     if (nstages > kLinMaxStages) nstages = kLinMaxStages;
     if (nstages < 2) MK36_FAIL(MK36_ERR_UNSUPPORTED, "linear_decode: shapes do not fit in shared memory");
     p.nstages = nstages;
-    const size_t smem_bytes = (size_t)p.off_ring + (size_t)nstages * p.stage_bytes;
+    const size_t smem_bytes = (size_t)p.off_ring + (size_t)nstages * stage_bytes;
 
-    const void* kernel = (a->dtype == MK36_BF16) ? (const void*)linear_decode_kernel<__nv_bfloat16> : (const void*)linear_decode_kernel<__half>;
+    const void* kernel = (a->dtype == MK36_BF16)
+                             ? (mma ? (const void*)linear_decode_kernel<__nv_bfloat16, true> : (const void*)linear_decode_kernel<__nv_bfloat16, false>)
+                             : (mma ? (const void*)linear_decode_kernel<__half, true> : (const void*)linear_decode_kernel<__half, false>);
     {
         const int rc = ensure_dynamic_smem(kernel, smem_bytes);
         if (rc != MK36_OK) return rc;
