@@ -149,7 +149,7 @@ __device__ __forceinline__ unsigned long long argmax_key(float v, int row) {
 
 // MMA: three to eight tokens on tensor-core instructions (tokens are the eight columns of the tile).  A kernel of its own:
 // decided at run time inside one kernel, the same choice cost the calls of one and two tokens 1 to 7 % (35B q|k|v
-// projection, two tokens: 14.5 us that way, 12.4 this way; LM head, one token: 198.7 and 191.3).
+// projection, two tokens: 14.5 us that way, 13.1 this way; LM head, one token: 198.7 and 191.3).
 template <typename T, bool MMA>
 __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const LinearParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -212,7 +212,10 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
                 if (++kstep == ksteps) { kstep = 0; first += p.rows; }
                 if (++stage == R) { stage = 0; ++use; }
             }
-            if (lane == 0 && !ok) atomicCAS(&p.ctl->status, 0, kStatusLinearProducer);
+            if (lane == 0) {
+                if (!ok) atomicCAS(&p.ctl->status, 0, kStatusLinearProducer);
+                ring_drain(full_bar, R, stage, use);
+            }
             return;
         }
         if (lane != 0) return;
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
             if (++stage == R) { stage = 0; ++use; }
         }
         if (!ok) atomicCAS(&p.ctl->status, 0, kStatusLinearProducer);
-        // consumers wait on every barrier that was armed, so no copy is in flight when the CTA leaves
+        ring_drain(full_bar, R, stage, use);
         return;
     }
 
@@ -417,7 +420,9 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
 #pragma unroll 1
     for (int k = 0; k < my_chunks; ++k) {
         ok = mbar_wait(&full_bar[stage], (unsigned)use & 1u, &s_abort);
-        if (!ok) break;
+        // on the tensor-core path a warp whose wait has run out comes to every tile's barrier like the others: the barrier
+        // has no limit, and they may be some tiles from giving up
+        if (!ok && (!MMA || dead)) break;
         if (tid == 0 && cta == 0 && k == 1) trace_stamp(p.ctl, 2);
         if (dead) {  // only drain the copies
             __syncwarp();
@@ -436,17 +441,19 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
             // the tile's last stage; then the eight partial tiles meet in shared memory (two buffers, so one block-wide
             // barrier per tile) and 128 threads finish one output each.
             const int g = lane >> 2, t = lane & 3;
-            const int k0 = kstep * p.kc;
-            const int nsl = min(p.kc, p.K - k0) >> 8;  // 32-wide slices per warp
-            const int kw = warp * nsl * 32 + 8 * t;
-            const T* alo = sbase + (size_t)min(g, count - 1) * (p.kc + kLinPad) + kw;  // rows beyond the tile repeat its last one: not stored
-            const T* ahi = sbase + (size_t)min(g + 8, count - 1) * (p.kc + kLinPad) + kw;
-            const T* bx = xs + (size_t)g * xstride + k0 + kw;
+            if (ok) {
+                const int k0 = kstep * p.kc;
+                const int nsl = min(p.kc, p.K - k0) >> 8;  // 32-wide slices per warp
+                const int kw = warp * nsl * 32 + 8 * t;
+                const T* alo = sbase + (size_t)min(g, count - 1) * (p.kc + kLinPad) + kw;  // rows beyond the tile repeat its last one: not stored
+                const T* ahi = sbase + (size_t)min(g + 8, count - 1) * (p.kc + kLinPad) + kw;
+                const T* bx = xs + (size_t)g * xstride + k0 + kw;
 #pragma unroll 4
-            for (int sl = 0; sl < nsl; ++sl) mma_slice32<T>(d0, d1, lds128(alo + 32 * sl), lds128(ahi + 32 * sl), lds128(bx + 32 * sl));
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty_bar[stage]);  // the weights of this stage have been read
-            if (++stage == R) { stage = 0; ++use; }
+                for (int sl = 0; sl < nsl; ++sl) mma_slice32<T>(d0, d1, lds128(alo + 32 * sl), lds128(ahi + 32 * sl), lds128(bx + 32 * sl));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty_bar[stage]);  // the weights of this stage have been read
+                if (++stage == R) { stage = 0; ++use; }
+            }
             if (++kstep < ksteps) continue;
             float* red = reinterpret_cast<float*>(smem + p.off_red) + (size_t)buffer * (kLinConsumerWarps * kLinMmaRows * 8);
             float* mine = red + (size_t)warp * (kLinMmaRows * 8);
@@ -458,7 +465,7 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
             tile_first += p.rows;
             buffer ^= 1;
             named_barrier(1, kLinConsumerThreads);
-            if (tid < kLinMmaRows * 8) {
+            if (tid < kLinMmaRows * 8 && *(volatile int*)&s_abort == 0) {  // set before the barrier by a warp that lacks its share
                 const int row = tid >> 3, tok = tid & 7;
                 if (row < count && tok < p.ntok) {
                     float v = 0.0f;
@@ -551,22 +558,20 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_decode_kernel(const Lin
         slot += count;
         while (slot >= kLinConsumerWarps) slot -= kLinConsumerWarps;
     }
-    if (!ok) {
-        atomicCAS(&p.ctl->status, 0, kStatusLinearConsumer);
-        return;
-    }
+    if (!ok || *(volatile int*)&s_abort != 0) atomicCAS(&p.ctl->status, 0, kStatusLinearConsumer);
     if (dead) return;
     if (tid == 0 && cta == ncta - 1) trace_stamp(p.ctl, 3);
+    if (!p.argmax) return;  // nothing crosses CTAs: the output rows are stored, the CTA is done
 
     // ---- arg-max: CTA-wide maxima first ----
-    if (p.argmax && MMA) {
+    if (MMA) {
         if (tid < kLinMmaRows * 8 && best0 != 0ull) atomicMax(&s_best[tid & 7], best0);
-    } else if (p.argmax && lane < 16) {
+    } else if (lane < 16) {
         if (best0 != 0ull) atomicMax(&s_best[lane & 3], best0);
         if (best1 != 0ull) atomicMax(&s_best[4 + (lane & 3)], best1);
     }
-    if (!p.argmax) return;  // nothing crosses CTAs: the output rows are stored, the CTA is done
-    named_barrier(1, kLinConsumerThreads);
+    named_barrier(1, kLinConsumerThreads);  // warps that gave up come here too
+    if (*(volatile int*)&s_abort != 0) return;
     if (tid < p.ntok && s_best[tid] != 0ull) atomicMax(&p.ctl->best[tid], s_best[tid]);
     if (tid == 0) {
         __threadfence();

@@ -66,7 +66,7 @@ def test_attention_block_reads_caches_longer_than_the_context(heads, position, c
     assert torch.equal(dev["k_cache"][:, rest].cpu(), cache["k_cache"][:, rest]) and torch.equal(dev["v_cache"][:, rest].cpu(), cache["v_cache"][:, rest])
 
 
-@pytest.mark.parametrize("kernel", ["dense_tiles"])
+@pytest.mark.parametrize("kernel", ["dense_tiles", "projection_tiles", "projection_tiles_argmax", "projection_rows_argmax"])
 def test_ring_fed_kernels_leave_together_when_their_waits_fail(kernel, cuda_device):
     """Behind a wait that has given up (made on the host side: a barrier that expects an arrival nobody makes) the status is
     still reported and nothing is stored; with the workspace initialised again the same call gives the operator's result."""
