@@ -139,12 +139,24 @@ __device__ __forceinline__ void attention_merge_few_splits(const AttnParams& p, 
                     for (int i = 0; i < 2; ++i) ms[i] = (ms[i] == -INFINITY) ? 0.0f : __expf(ms[i] - mm);  // now the splits' weights
                     lsum = warp_sum(fmaf(ms[0], ls[0], ms[1] * ls[1]));
                 }
+                // eight chains of four splits and a tree over them: one chain through all splits is further from the exact sum
+                // than the merge above (49 splits: 1.4e-7 against 8.3e-8, fp32 sums of drawn partials; this way 7.5e-8)
+                float4 part[8];
 #pragma unroll
                 for (int s = 0; s < 32; ++s) {
                     const float sc = __shfl_sync(kFullMask, ms[j], s);
-                    acc[0] = fmaf(sc, v[s].x, acc[0]); acc[1] = fmaf(sc, v[s].y, acc[1]);
-                    acc[2] = fmaf(sc, v[s].z, acc[2]); acc[3] = fmaf(sc, v[s].w, acc[3]);
+                    float4& a = part[s & 7];
+                    if (s < 8) a = make_float4(sc * v[s].x, sc * v[s].y, sc * v[s].z, sc * v[s].w);
+                    else a = make_float4(fmaf(sc, v[s].x, a.x), fmaf(sc, v[s].y, a.y), fmaf(sc, v[s].z, a.z), fmaf(sc, v[s].w, a.w));
                 }
+#pragma unroll
+                for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+                    for (int i = 0; i < w; ++i) {
+                        part[i].x += part[i + w].x; part[i].y += part[i + w].y;
+                        part[i].z += part[i + w].z; part[i].w += part[i + w].w;
+                    }
+                acc[0] += part[0].x; acc[1] += part[0].y; acc[2] += part[0].z; acc[3] += part[0].w;
             }
         }
         T* o = out + (size_t)bh * p.D + dc * 128 + 4 * lane;

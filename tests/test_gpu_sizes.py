@@ -114,3 +114,17 @@ def test_ring_fed_kernels_leave_together_when_their_waits_fail(kernel, cuda_devi
         else:
             assert rc == 0 and status.value == 0
             assert torch.equal(out, expect) and (best is None or torch.equal(best, expect_best))
+
+
+@pytest.mark.parametrize("shape,dtype", [((1, 4, 2, 128, 16), torch.bfloat16), ((1, 4, 2, 128, 16 * 33), torch.float16), ((1, 16, 2, 256, 16 * 64), torch.bfloat16),
+                                         ((1, 4, 2, 128, 16 * 64 + 1), torch.bfloat16), ((5, 16, 2, 256, 611), torch.float16), ((4, 8, 2, 64, 300), torch.bfloat16)])
+def test_attention_merges_at_the_split_counts_where_they_change(shape, dtype, cuda_device):
+    """One split, 33 (a second round of the channel-wise merge), 64 (its last) and 65 (the merge over lanes); several batch
+    items; head_dim 64, which the channel-wise merge does not take."""
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import synthetic as syn
+    from oracle import decode_oracle as oracle
+
+    t = syn.attention_tensors(*shape, seed=shape[4], dtype=dtype)
+    got = mk.full_attention_decode(mk.FullAttentionInputs(*(t[n].to(cuda_device) for n in ("q", "k_cache", "v_cache")))).cpu()
+    assert_output_parity(got, oracle.full_attention_decode(t["q"], t["k_cache"], t["v_cache"]), what=f"merge {shape}")
