@@ -19,6 +19,11 @@
 //            so that a warp's activation fragments serve three stages
 //   combine  in shared memory; residual, rounding, store (or the cross-GPU exchange)
 //
+// Sums: a stage's products are one chain of MMAs from zero, and the stages are added up in fp32.  As one chain over all
+// stages, f16 at an eighth of the width was further from the 64-bit sum than the register-staged kernel (relative error
+// 1.15e-6 against 0.97e-6); this way 4.1e-7, and bf16 at the whole width 2.5e-6 against 6.4e-6.  It costs 1 % (27B, four
+// tokens 109.1 -> 110.5 us).
+//
 // Fragment conventions: mk36_mma.cuh.  Ring protocol: mk36_ring.cuh, every consumer warp observes and
 // releases every stage.
 #include "mk36_comm.cuh"
@@ -224,9 +229,12 @@ __global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const De
             const T* ahi = sbase + (size_t)(p.pa + rl) * (p.kca + kDtPad) + 8 * t;
             const T* bx = xs + (size_t)g * xstride + (size_t)k * p.kca + 8 * t;
             const int width = min(p.kca, p.H - k * p.kca);
+            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
-            for (int c = 32 * warp; c < width; c += 32 * kDtWarps) mma_slice32<T>(d0, d1, lds128(alo + c), lds128(ahi + c), lds128(bx + c));
+            for (int c = 32 * warp; c < width; c += 32 * kDtWarps) mma_slice32<T>(s0, s1, lds128(alo + c), lds128(ahi + c), lds128(bx + c));
             release();
+            add_tile(d0, s0);
+            add_tile(d1, s1);
         }
         // The warps' shares of the tile meet; two buffers, so one barrier per tile.  A warp whose wait has run out comes to
         // every tile's barrier like the others: the barrier has no limit, and they may be some tiles from giving up.  What
@@ -305,16 +313,19 @@ __global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const De
                         const T* sbase = reinterpret_cast<const T*>(ring + (size_t)stage * kDtStageBytes) + 8 * t;
                         const T* alo = sbase + (size_t)min(g, count - 1) * (p.kcc + kDtPad);
                         const T* ahi = sbase + (size_t)min(g + 8, count - 1) * (p.kcc + kDtPad);
+                        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                         for (int s = 0; s < kDtDownSlices; ++s) {
                             const int c = 32 * (warp + s * kDtWarps);
                             if (c < width) {
                                 const uint4 a = lds128(alo + c), b = lds128(ahi + c);
-                                mma_slice32<T>(acc[i][0], acc[i][1], a, b, bh[s]);
-                                mma_slice32<T>(acc[i][0], acc[i][1], a, b, bl[s]);
+                                mma_slice32<T>(s0, s1, a, b, bl[s]);
+                                mma_slice32<T>(s0, s1, a, b, bh[s]);
                             }
                         }
                         release();
+                        add_tile(acc[i][0], s0);
+                        add_tile(acc[i][1], s1);
                     }
                 }
             }

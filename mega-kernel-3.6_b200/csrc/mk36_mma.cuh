@@ -37,6 +37,13 @@ __device__ __forceinline__ void mma_slice32(float (&d0)[4], float (&d1)[4], cons
     mma_16816<T>(d1, a_lo.z, a_hi.z, a_lo.w, a_hi.w, b.z, b.w);
 }
 
+// a += b: the end of a short chain of MMAs.  The tensor core cuts what it adds to an accumulator off where an fp32 addition
+// rounds, so long sums are chains of a few MMAs from zero that are added up here.
+__device__ __forceinline__ void add_tile(float (&a)[4], const float (&b)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] += b[i];
+}
+
 #endif  // __CUDACC__
 
 }  // namespace mk36

@@ -128,3 +128,35 @@ def test_attention_merges_at_the_split_counts_where_they_change(shape, dtype, cu
     t = syn.attention_tensors(*shape, seed=shape[4], dtype=dtype)
     got = mk.full_attention_decode(mk.FullAttentionInputs(*(t[n].to(cuda_device) for n in ("q", "k_cache", "v_cache")))).cpu()
     assert_output_parity(got, oracle.full_attention_decode(t["q"], t["k_cache"], t["v_cache"]), what=f"merge {shape}")
+
+
+def _exactly_normalised(batch, hidden, dtype, gen, device):
+    """x of +-1 and a norm weight: with eps 0 the normalised token is x * weight without any rounding."""
+    x = (torch.randint(0, 2, (batch, hidden), generator=gen) * 2 - 1).to(dtype).to(device)
+    return x, (torch.randn(hidden, generator=gen) * 0.6 + 1.0).to(dtype).to(device)
+
+
+def _error(got, exact):
+    return float((got.double() - exact).norm() / exact.norm())
+
+
+@pytest.mark.parametrize("batch,intermediate,dtype", [(2, 2176, torch.float16), (8, 2176, torch.float16), (8, 2176, torch.bfloat16), (3, 4352, torch.bfloat16)],
+                         ids=lambda v: str(v).replace("torch.", ""))
+def test_dense_tiles_are_no_further_from_the_exact_sum_than_the_register_staged_kernel(batch, intermediate, dtype, cuda_device):
+    """fp32 partial outputs of both kernels against 64-bit sums of the same inputs."""
+    from mega_kernel_qwen36 import cabi, ops
+
+    gen = torch.Generator().manual_seed(intermediate + batch)
+    hidden = 5120
+    x, norm = _exactly_normalised(batch, hidden, dtype, gen, cuda_device)
+    gate, up, down = ((torch.randn(*s, generator=gen) * 0.02).to(dtype).to(cuda_device) for s in ((intermediate, hidden), (intermediate, hidden), (hidden, intermediate)))
+    n = (x * norm).double()
+    exact = (torch.nn.functional.silu(n @ gate.double().T) * (n @ up.double().T)) @ down.double().T
+    errors = {}
+    for tiles in (0, 1):
+        cabi.check(cabi.load().mk36_set_option(b"dense_tiles", tiles))
+        try:
+            errors[tiles] = _error(ops._C.dense_ffn_decode_partial(x, norm, gate, up, down, 0.0), exact)
+        finally:
+            cabi.check(cabi.load().mk36_set_option(b"dense_tiles", 1))
+    assert errors[1] <= errors[0], errors
