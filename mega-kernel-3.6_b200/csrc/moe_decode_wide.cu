@@ -11,8 +11,16 @@
 // covers whole 128-byte lines: 16-byte loads took 204 against 188 us.  Twelve warps: 16 with 128 registers
 // took 193, 8 with twice the slices in flight 202.
 //
-// Hidden 2048, 256 experts of width 512, top 8, bf16, 32 tokens: 314 us as four launches of the batch
-// kernel, 204 here (1.03 GB: 5.05 TB/s).
+// Hidden 2048, 256 experts of width 512, top 8, bf16, 32 tokens: 315 us as four launches of the batch
+// kernel, 205 here (1.03 GB: 5.0 TB/s).
+//
+// Sums: the tensor core cuts off where an fp32 addition rounds.  As one chain of MMAs over a whole sum the
+// fp32 output was eight times as far from the 64-bit sum as the batch kernel's, which rounds every addition
+// (relative error 1.25e-6 against 1.6e-7).  So a 32-wide slice is a chain of its own from zero, slices are
+// added up in fp32, and what is done a few times per value (the four shares of a gate/up tile, silu(g) * u
+// behind the exponential, the slots of a token) in fp64: 1.6e-7 as well, at 3 % (32 tokens 198 -> 205 us).
+// Taken back: pieces of eight products (no closer, 8 % slower); even and odd accumulators or fp64 in the down
+// sums too (1.55e-7 and 1.45e-7, 217 and 219 us).
 //
 //   phase 0   every CTA normalises all tokens into shared memory and dots them with its one or two
 //             router rows (fp32 FMA: the choice of experts does not depend on the kernel) | arrive 1
@@ -83,6 +91,9 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16& hi, __nv_bfloat16
     lo = __float2bfloat16_rn(finite ? r - m : 0.0f);
 }
 
+// silu(g) * u with one rounding behind the exponential
+__device__ __forceinline__ float swiglu_exact(float g, float u) { return (float)((double)g * u / (1.0 + expf(-g))); }
+
 // Gate/up units [first, end) in steps of `step`, tile units of the entries from `entry0`, by the four warps of a quad.
 struct WideGateUp {
     const __nv_bfloat16* gate;
@@ -120,6 +131,7 @@ __device__ __forceinline__ void wide_gate_up(const WideGateUp w, int first, int 
 #pragma unroll 1
     for (int u = first; u < end; u += step) {
         float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
+        float d2[4] = {0.f, 0.f, 0.f, 0.f}, d3[4] = {0.f, 0.f, 0.f, 0.f};
         const T* bcol = xs + (size_t)ent_tok[entry * kWdCols + g] * x_stride + koff;
 #pragma unroll 1
         for (int r = 0; r < R; ++r) {
@@ -131,8 +143,13 @@ __device__ __forceinline__ void wide_gate_up(const WideGateUp w, int first, int 
             const T* nb = w.up + off;
 #pragma unroll
             for (int j = 0; j < kWdAhead; j += 2) {
-                mma_slice32<T>(d0, d1, qa[j], qb[j], lds128(bcol + 32 * j));
-                mma_slice32<T>(d0, d1, qa[j + 1], qb[j + 1], lds128(bcol + 32 * j + 8));
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma_slice32<T>(s0, s1, qa[j + q], qb[j + q], lds128(bcol + 32 * j + 8 * q));
+                    add_tile(q ? d2 : d0, s0);
+                    add_tile(q ? d3 : d1, s1);
+                }
                 if (more) {
                     ld_stream_2u4(na + 32 * j, qa[j], qa[j + 1]);
                     ld_stream_2u4(nb + 32 * j, qb[j], qb[j + 1]);
@@ -140,18 +157,22 @@ __device__ __forceinline__ void wide_gate_up(const WideGateUp w, int first, int 
             }
             bcol += 32 * kWdAhead;
         }
+        add_tile(d0, d2);
+        add_tile(d1, d3);
         // the quad's four shares of the tile; the warps take turns at finishing one.  Two buffers: a warp that
         // reads this one has left it before it arrives at the next unit's barrier.
         float4* mine = part + (size_t)((parity * kWdQuads + quad) * kWdQuadWarps) * 32;
         mine[kpart * 32 + lane] = make_float4(d0[0] + d1[0], d0[1] + d1[1], d0[2] + d1[2], d0[3] + d1[3]);
         named_barrier(1 + quad, kWdQuadWarps * 32);
         if (kpart == turn) {
-            float4 v = mine[lane];
+            const float4 v0 = mine[lane];
+            double vx = v0.x, vy = v0.y, vz = v0.z, vw = v0.w;
 #pragma unroll
             for (int q = 1; q < kWdQuadWarps; ++q) {
                 const float4 o = mine[q * 32 + lane];
-                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+                vx += o.x; vy += o.y; vz += o.z; vw += o.w;
             }
+            const float4 v = make_float4((float)vx, (float)vy, (float)vz, (float)vw);
             int e_unused, tile;
             fdivmod(u, w.tiles, e_unused, tile);
             const int ch = tile * 8 + g;
@@ -160,7 +181,7 @@ __device__ __forceinline__ void wide_gate_up(const WideGateUp w, int first, int 
                 const int pair = ent_pair[entry * kWdCols + 2 * t + c];
                 if (pair >= 0) {
                     T hi, mid, lo;
-                    split3(c == 0 ? silu(v.x) * v.z : silu(v.y) * v.w, hi, mid, lo);
+                    split3(c == 0 ? swiglu_exact(v.x, v.z) : swiglu_exact(v.y, v.w), hi, mid, lo);
                     T* dst = w.act + (size_t)(pair - w.pair0) * 3 * w.I + ch;
                     dst[0] = hi;
                     dst[w.I] = mid;
@@ -464,9 +485,12 @@ __global__ void __launch_bounds__(kWdThreads, 1) moe_decode_wide_kernel(const Mo
                 for (int j = 0; j < kWdDownAhead; j += 2) {
 #pragma unroll
                     for (int q = 0; q < 2; ++q) {
-                        mma_slice32<T>(d0, d1, wa[j + q], wb[j + q], fl[q]);
-                        mma_slice32<T>(d0, d1, wa[j + q], wb[j + q], fm[q]);
-                        mma_slice32<T>(d0, d1, wa[j + q], wb[j + q], fh[q]);
+                        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+                        mma_slice32<T>(s0, s1, wa[j + q], wb[j + q], fl[q]);
+                        mma_slice32<T>(s0, s1, wa[j + q], wb[j + q], fm[q]);
+                        mma_slice32<T>(s0, s1, wa[j + q], wb[j + q], fh[q]);
+                        add_tile(d0, s0);
+                        add_tile(d1, s1);
                         if (j + 2 < kWdDownAhead) fetch_act(q, arow == nullptr ? arow : arow + 32 * (j + 2) + 8 * q, len);
                         else if (more) fetch_act(q, nact == nullptr ? nact : nact + 8 * q, nlen);
                     }
@@ -496,14 +520,15 @@ __global__ void __launch_bounds__(kWdThreads, 1) moe_decode_wide_kernel(const Mo
     for (int item = tid; item < p.ntok * 16; item += kWdThreads) {
         const int b = item >> 4, j = item & 15;
         if (j < hr) {
-            float v = 0.0f;
+            double vd = 0.0;
 #pragma unroll 4
             for (int k = 0; k < p.K; ++k) {
                 const int pair = b * kWdSlots + k;
                 const int e = s_pair_e[pair];
-                if (e >= p.expert_base && e < p.expert_base + p.local_experts) v = fmaf(s_pair_w[pair], part_out[pair * p.hr_max + j], v);
+                if (e >= p.expert_base && e < p.expert_base + p.local_experts) vd = fma((double)s_pair_w[pair], (double)part_out[pair * p.hr_max + j], vd);
             }
-            if (p.Is > 0) v += part_out[(kWdPairs + b) * p.hr_max + j];
+            if (p.Is > 0) vd += part_out[(kWdPairs + b) * p.hr_max + j];
+            const float v = (float)vd;
             const size_t o = (size_t)b * H + h0 + j;
             if (p.partial_out) p.partial_out[o] = v;
             else p.out[o] = from_float<T>(p.add_residual ? v + to_float<T>(p.x[o]) : v);
