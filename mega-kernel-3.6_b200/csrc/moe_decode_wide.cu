@@ -195,7 +195,34 @@ __device__ __forceinline__ void wide_gate_up(const WideGateUp w, int first, int 
     }
 }
 
-__global__ void __launch_bounds__(kWdThreads, 1) moe_decode_wide_kernel(const MoeWideParams p) {
+// The elements of a warp's down products that came out as NaN, once more from the activations' values instead of their
+// terms: an infinite weight times a term that is zero is a NaN where the activation itself gives an infinity.
+static __device__ __noinline__ void wide_down_again(const MoeWideParams& p, float* part_out, const int* ent_e, const short* ent_pair, int entries, int nsh,
+                                                    int h0, int hr, int warp, int lane) {
+    __syncwarp();
+    for (int i = warp; i < entries; i += kWdWarps) {
+        const int len = i < nsh ? p.Is : p.I;
+        const __nv_bfloat16* rows = (i < nsh ? p.sdown : p.edown + (size_t)(ent_e[i] - p.expert_base) * p.H * p.I) + (size_t)h0 * len;
+        for (int c = 0; c < kWdCols; ++c) {
+            const int pair = ent_pair[i * kWdCols + c];
+            if (pair < 0) continue;
+            const __nv_bfloat16* act = pair >= kWdPairs ? p.sact + (size_t)(pair - kWdPairs) * 3 * p.Is : p.act + (size_t)pair * 3 * p.I;
+            for (int r = 0; r < hr; ++r) {
+                float* at = part_out + pair * p.hr_max + r;
+                if (!isnan(*at)) continue;  // the same for the whole warp
+                float sum = 0.0f;
+                for (int k = lane; k < len; k += 32) {
+                    const float a = (to_float(__ldcg(act + k)) + to_float(__ldcg(act + len + k))) + to_float(__ldcg(act + 2 * len + k));
+                    sum = fmaf(a, to_float(rows[(size_t)r * len + k]), sum);
+                }
+                sum = warp_sum(sum);
+                if (lane == 0) *at = sum;
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kWdThreads, 1) moe_decode_wide_kernel(const __grid_constant__ MoeWideParams p) {
     using T = __nv_bfloat16;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_flag;
@@ -465,6 +492,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) moe_decode_wide_kernel(const Mo
             fetch_act(0, arow, len);
             fetch_act(1, arow == nullptr ? arow : arow + 8, len);
         }
+        bool odd = false;  // an element of this warp came out as NaN
 #pragma unroll 1
         for (; i < entries; i += kWdWarps) {
             float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};
@@ -502,16 +530,19 @@ __global__ void __launch_bounds__(kWdThreads, 1) moe_decode_wide_kernel(const Mo
                 arow = nact;
             }
             // rows g and g + 8, columns 2t and 2t + 1
+            add_tile(d0, d1);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 const int pair = ent_pair[i * kWdCols + 2 * t + c];
                 if (pair >= 0) {
-                    if (vlo) part_out[pair * p.hr_max + g] = d0[c] + d1[c];
-                    if (vhi) part_out[pair * p.hr_max + g + 8] = d0[2 + c] + d1[2 + c];
+                    if (vlo) part_out[pair * p.hr_max + g] = d0[c];
+                    if (vhi) part_out[pair * p.hr_max + g + 8] = d0[2 + c];
+                    odd |= (vlo && isnan(d0[c])) || (vhi && isnan(d0[2 + c]));
                 }
             }
             len = nlen;
         }
+        if (__any_sync(kFullMask, odd)) wide_down_again(p, part_out, ent_e, ent_pair, entries, nsh, h0, hr, warp, lane);
     }
     if (tracer) trace_stamp(p.ctl, 7);
     __syncthreads();

@@ -189,3 +189,24 @@ def test_moe_wide_kernel_is_as_close_to_the_exact_sum_as_the_batch_kernel(batch,
         for slot, e in enumerate(idx[b].tolist()):
             exact[b] += mix[b, slot] * ((silu(n[b] @ gate[e].double().T) * (n[b] @ up[e].double().T)) @ down[e].double().T)
     assert _error(got[9], exact) <= 1.1 * _error(got[0], exact)
+
+
+def test_moe_wide_kernel_keeps_infinite_weights(cuda_device):
+    """One infinite down weight in every other output row, at another channel in each: the output is an infinity of the
+    activation's sign, as the batch kernel's is, also where a term that the activation is split into is zero."""
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import cabi, synthetic as syn
+
+    t = {k: v.to(cuda_device) for k, v in syn.moe_tensors(syn.MOE_35B_A3B, 32, 3, torch.bfloat16).items()}
+    rows = torch.arange(0, t["shared_down"].shape[0], 2, device=cuda_device)
+    t["shared_down"][rows, (rows * 7) % t["shared_down"].shape[1]] = float("inf")
+    weights = mk.MoeWeights(*[t[f] for f in syn.MOE_WEIGHT_FIELDS])
+    got = mk.moe_decode(t["x"], weights)[0].float()
+    cabi.check(cabi.load().mk36_set_option(b"moe_wide", 0))
+    try:
+        want = mk.moe_decode(t["x"], weights)[0].float()
+    finally:
+        cabi.check(cabi.load().mk36_set_option(b"moe_wide", 9))
+    assert bool(want[:, rows].isinf().all())
+    assert torch.equal(got[:, rows], want[:, rows])
+    assert_output_parity(got[:, 1::2].cpu(), want[:, 1::2].cpu(), what="rows without an infinite weight")
