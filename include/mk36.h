@@ -352,7 +352,8 @@ MK36_API int mk36_linear_attention_decode(const mk36_linear_attention_args* args
  * step t reads its q/k/v, updates the state and writes out[t]; the state is read from `state` once and
  * written to `new_state` once (they may be the same buffer).  decay_per_step / beta_per_step are
  * optional fp32 [steps, batch, value_heads] gates (NULL: the scalar `decay`, beta 1).  Outputs
- * and final state are bit-identical to `steps` calls of mk36_linear_attention_decode.  The reference's
+ * and final state are bit-identical to `steps` calls of mk36_linear_attention_decode.  A value_dim that is not a multiple
+ * of four, a key_dim above 256 or a state that is not 16-byte aligned takes one launch per step instead.  The reference's
  * operator is one step per call (mega_kernel_qwen36/ops.py:377-386), so this entry point has no
  * counterpart there; it exists because a one-step call has to move the whole state (2 MiB per
  * batch row at the 35B-A3B shape) through HBM twice per token. */

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kLinThreads) linear_attention_kernel(const Lin
 }
 
 // ---------------------------------------------------------------------------------------------
-// The strip kernels: value_dim and key_dim multiples of four, key_dim <= 256, aligned tensors.
+// The strip kernels: value_dim and key_dim multiples of four, key_dim <= 256, aligned states.
 //
 // A warp owns 16 value columns of one (batch, value head) state matrix: lane = (row group g = lane / 4,
 // column quad c = lane % 4), and a thread keeps columns 4c .. 4c + 3 of the rows 32 i + 4 g + j (j < 4),
@@ -169,6 +169,13 @@ __device__ __forceinline__ float4 quad_floats(const Quad<float>& r) {
     return make_float4(__uint_as_float(r.raw.x), __uint_as_float(r.raw.y), __uint_as_float(r.raw.z), __uint_as_float(r.raw.w));
 }
 
+// the same where the address may be aligned to one element only
+template <bool ALIGNED, typename T>
+__device__ __forceinline__ float4 load_floats(const T* p) {
+    if constexpr (ALIGNED) return quad_floats(load_quad(p));
+    else return make_float4(to_float<T>(p[0]), to_float<T>(p[1]), to_float<T>(p[2]), to_float<T>(p[3]));
+}
+
 // Two fp32 values per instruction (each rounded on its own, as the scalar instructions round).
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack2(float a, float b) {
@@ -198,6 +205,15 @@ template <typename T>
 __device__ __forceinline__ void cp_async_quad(T* dst, const T* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "n"(4 * (int)sizeof(T)) : "memory");
 }
+template <bool ALIGNED, typename T>
+__device__ __forceinline__ void stage_quad(T* dst, const T* src) {
+    if constexpr (ALIGNED) {
+        cp_async_quad(dst, src);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[i] = src[i];
+    }
+}
 __device__ __forceinline__ void cp_async4(void* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
@@ -214,10 +230,12 @@ __device__ __forceinline__ float reduce_columns(const float (&o)[4], int lane) {
     return c + __shfl_xor_sync(kFullMask, c, 4);
 }
 
-// NQ: row quads of a thread (4: key_dim <= 128, 8: <= 256).  FULL: key_dim is exactly 32 NQ.
+// NQ: row quads of a thread (4: key_dim <= 128, 8: <= 256).  FULL: key_dim is exactly 32 NQ.  ALIGNED: q, k and v are aligned
+// to four elements; where they are not they are read element by element, and everything else is the same (64 steps, eight
+// tokens, 32 heads of 128 x 128: 59 us aligned, 71 not, 525 as 64 launches).
 //
 // One step: a stream through registers; all of a thread's loads are in flight before anything waits.
-template <typename T, int NQ, bool FULL>
+template <typename T, int NQ, bool FULL, bool ALIGNED>
 __global__ void __launch_bounds__(kStripThreads) linear_strip_kernel(const LinParams p) {
     extern __shared__ __align__(16) float s_dyn[];  // k[Dk], q[Dk]
     const int slices = (p.Dv + kStripCols - 1) / kStripCols;
@@ -239,7 +257,7 @@ __global__ void __launch_bounds__(kStripThreads) linear_strip_kernel(const LinPa
         }
     const size_t qk = ((size_t)b * p.Hk + hk) * p.Dk;
     float4 vv = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live) vv = quad_floats(load_quad(static_cast<const T*>(p.v) + ((size_t)b * p.Hv + h) * p.Dv + col0));
+    if (live) vv = load_floats<ALIGNED>(static_cast<const T*>(p.v) + ((size_t)b * p.Hv + h) * p.Dv + col0);
     const float decay = p.decay_ph ? p.decay_ph[(size_t)b * p.Hv + h] : p.decay;
     if (p.beta_ph) {
         const float beta = p.beta_ph[(size_t)b * p.Hv + h];
@@ -248,7 +266,7 @@ __global__ void __launch_bounds__(kStripThreads) linear_strip_kernel(const LinPa
     for (int i = tid; i < p.Dk / 2; i += kStripThreads) {  // quads of k, then of q
         const bool is_k = i < p.Dk / 4;
         const T* src = static_cast<const T*>(is_k ? p.k : p.q) + qk + 4 * (is_k ? i : i - p.Dk / 4);
-        *reinterpret_cast<float4*>(s_dyn + 4 * i) = quad_floats(load_quad(src));
+        *reinterpret_cast<float4*>(s_dyn + 4 * i) = load_floats<ALIGNED>(src);
     }
     __syncthreads();
     float even[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};
@@ -290,7 +308,7 @@ __global__ void __launch_bounds__(kStripThreads) linear_strip_kernel(const LinPa
 // Measured at 64 steps, eight tokens, 32 heads of 128 x 128: 59 us (about 34 us of it is the FP32 pipe of an average
 // SM, the rest what the busiest scheduler has above the average and its other instructions); the kernel before
 // it, two barriers of 256 threads and a sum through shared memory per step, took 260 us.
-template <typename T, int NQ, bool FULL>
+template <typename T, int NQ, bool FULL, bool ALIGNED>
 __global__ void __launch_bounds__(kStripThreads, NQ == 4 ? 7 : 4) linear_strip_steps_kernel(const LinStepsParams p) {
     extern __shared__ __align__(16) unsigned char s_raw[];  // [kStripAhead + 1][kStripChunk][k Dk | q Dk | v kStripCols | decay, beta]
     const int slices = (p.Dv + kStripCols - 1) / kStripCols;
@@ -340,12 +358,12 @@ __global__ void __launch_bounds__(kStripThreads, NQ == 4 ? 7 : 4) linear_strip_s
             const int idx = tid + r * kStripThreads;
             const int row = idx / kRowQuads, c = 4 * (idx % kRowQuads), step = step0 + (row >> 1);
             if (step < p.steps && (FULL || c < Dk))
-                cp_async_quad(reinterpret_cast<T*>(buf + (row >> 1) * stride) + (row & 1) * Dk + c, ((row & 1) ? q : k) + (size_t)step * qk_step + c);
+                stage_quad<ALIGNED>(reinterpret_cast<T*>(buf + (row >> 1) * stride) + (row & 1) * Dk + c, ((row & 1) ? q : k) + (size_t)step * qk_step + c);
         }
         {
             const int s = tid / kVQuads, c = 4 * (tid % kVQuads), step = step0 + s;
             if (s < kStripChunk && step < p.steps && slice * kStripCols + c < p.Dv)
-                cp_async_quad(reinterpret_cast<T*>(buf + s * stride) + 2 * Dk + c, v + (size_t)step * v_step + c);
+                stage_quad<ALIGNED>(reinterpret_cast<T*>(buf + s * stride) + 2 * Dk + c, v + (size_t)step * v_step + c);
         }
         if (tid < 2 * kStripChunk) {
             const float* gate = (tid & 1) ? p.beta_ps : p.decay_ps;
@@ -440,30 +458,155 @@ __global__ void __launch_bounds__(kStripThreads, NQ == 4 ? 7 : 4) linear_strip_s
         }
 }
 
-// Whether the strip kernels take a call.  Both the one-step and the multi-step entry point ask this, so
-// that their results agree bit for bit.
-bool strip_fits(int dtype, int key_dim, int value_dim, const void* q, const void* k, const void* v, const float* state, const float* new_state) {
-    const uintptr_t quad = dtype == MK36_F32 ? 15u : 7u;  // bytes of four elements, less one
-    const uintptr_t qkv = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v);
+// ---------------------------------------------------------------------------------------------
+// Several steps in one launch where key_dim is not a multiple of four, which the strips need.  The partition and the arithmetic of linear_attention_kernel, in the same order, so that T steps are
+// bit-identical to T of its launches; a thread keeps up to eight rows by four columns of the state in registers and the
+// next step's q, k, v are fetched, element by element, while the current step is computed.  Two block-wide barriers and a
+// sum through shared memory per step: four times the strips' time, but a launch per step passes the state through HBM
+// each time (64 steps, eight tokens, 32 heads of 126 x 128, bf16: 200 us, as 64 launches 653).
+// ---------------------------------------------------------------------------------------------
+constexpr int kLinStepRows = 8;  // state rows per thread: key_dim <= 8 * 32
+
+template <typename T>
+__global__ void __launch_bounds__(kLinThreads) linear_attention_steps_kernel(const LinStepsParams p) {
+    constexpr int VEC = 4;
+    constexpr int CT = kLinCols / VEC;     // 8 threads across the column slice
+    constexpr int RG = kLinThreads / CT;   // 32 row groups
+    extern __shared__ float s_dyn[];       // q[Dk], k[Dk]
+    __shared__ float s_red[RG][kLinCols + 1];
+    __shared__ float s_v[kLinCols];
+
+    const int slices = (p.Dv + kLinCols - 1) / kLinCols;
+    const int slice = blockIdx.x % slices;
+    const int bh = blockIdx.x / slices;
+    const int h = bh % p.Hv;
+    const int b = bh / p.Hv;
+    const int hk = h / (p.Hv / p.Hk);
+    const int tid = threadIdx.x;
+    const int ct = tid % CT, rg = tid / CT;
+    const int col0 = slice * kLinCols + ct * VEC;
+    const bool live = col0 < p.Dv;  // Dv % 4 == 0 on this path
+
+    float* s_q = s_dyn;
+    float* s_k = s_dyn + p.Dk;
+    const size_t qk_step = (size_t)p.B * p.Hk * p.Dk, v_step = (size_t)p.B * p.Hv * p.Dv, g_step = (size_t)p.B * p.Hv;
+    const T* q = static_cast<const T*>(p.q) + ((size_t)b * p.Hk + hk) * p.Dk;
+    const T* k = static_cast<const T*>(p.k) + ((size_t)b * p.Hk + hk) * p.Dk;
+    const T* v = static_cast<const T*>(p.v) + ((size_t)b * p.Hv + h) * p.Dv + slice * kLinCols;
+    T* out = static_cast<T*>(p.out) + ((size_t)b * p.Hv + h) * p.Dv + slice * kLinCols;
+    const size_t gidx = (size_t)b * p.Hv + h;
+
+    // the state slice of this thread: rows rg, rg + 32, ... x 4 columns
+    const size_t base = ((size_t)b * p.Hv + h) * p.Dk * p.Dv;
+    float4 st[kLinStepRows];
+#pragma unroll
+    for (int r = 0; r < kLinStepRows; ++r) {
+        const int kd = rg + r * RG;
+        st[r] = (live && kd < p.Dk) ? *reinterpret_cast<const float4*>(p.state + base + (size_t)kd * p.Dv + col0)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+
+    // software pipeline: thread i carries element i (and i + 256) of the next step's q and k, and
+    // the first 32 threads the next step's v slice
+    auto fetch = [&](int step, float (&nq)[2], float (&nk)[2], float& nv) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int i = tid + j * kLinThreads;
+            nq[j] = (i < p.Dk) ? to_float<T>(q[(size_t)step * qk_step + i]) : 0.0f;
+            nk[j] = (i < p.Dk) ? to_float<T>(k[(size_t)step * qk_step + i]) : 0.0f;
+        }
+        nv = (tid < kLinCols && slice * kLinCols + tid < p.Dv) ? to_float<T>(v[(size_t)step * v_step + tid]) : 0.0f;
+    };
+    float nq[2], nk[2], nv;
+    fetch(0, nq, nk, nv);
+
+    for (int step = 0; step < p.steps; ++step) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int i = tid + j * kLinThreads;
+            if (i < p.Dk) { s_q[i] = nq[j]; s_k[i] = nk[j]; }
+        }
+        if (tid < kLinCols) s_v[tid] = nv;
+        const float decay = p.decay_ps ? p.decay_ps[(size_t)step * g_step + gidx] : p.decay;
+        const float beta = p.beta_ps ? p.beta_ps[(size_t)step * g_step + gidx] : 1.0f;
+        __syncthreads();
+        if (step + 1 < p.steps) fetch(step + 1, nq, nk, nv);
+
+        float vv[VEC], o[VEC];
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            const float raw = s_v[ct * VEC + j];
+            vv[j] = p.beta_ps ? __fmul_rn(raw, beta) : raw;
+            o[j] = 0.0f;
+        }
+        if (live) {
+#pragma unroll
+            for (int r = 0; r < kLinStepRows; ++r) {
+                const int kd = rg + r * RG;
+                if (kd < p.Dk) {
+                    const float kk = s_k[kd], qq = s_q[kd];
+                    float4 n;
+                    n.x = __fadd_rn(__fmul_rn(st[r].x, decay), __fmul_rn(kk, vv[0]));
+                    n.y = __fadd_rn(__fmul_rn(st[r].y, decay), __fmul_rn(kk, vv[1]));
+                    n.z = __fadd_rn(__fmul_rn(st[r].z, decay), __fmul_rn(kk, vv[2]));
+                    n.w = __fadd_rn(__fmul_rn(st[r].w, decay), __fmul_rn(kk, vv[3]));
+                    st[r] = n;
+                    o[0] = fmaf(qq, n.x, o[0]);
+                    o[1] = fmaf(qq, n.y, o[1]);
+                    o[2] = fmaf(qq, n.z, o[2]);
+                    o[3] = fmaf(qq, n.w, o[3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) s_red[rg][ct * VEC + j] = o[j];
+        __syncthreads();
+        if (tid < kLinCols && slice * kLinCols + tid < p.Dv) {
+            float sum = 0.0f;
+#pragma unroll 8
+            for (int r = 0; r < RG; ++r) sum += s_red[r][tid];
+            out[(size_t)step * v_step + tid] = from_float<T>(sum);
+        }
+        // the next iteration's writes to s_q / s_k / s_v happen after everyone has passed the barrier
+        // above; its writes to s_red come after its own first barrier, i.e. after the sums were read
+    }
+
+#pragma unroll
+    for (int r = 0; r < kLinStepRows; ++r) {
+        const int kd = rg + r * RG;
+        if (live && kd < p.Dk) *reinterpret_cast<float4*>(p.new_state + base + (size_t)kd * p.Dv + col0) = st[r];
+    }
+}
+
+// Whether the strip kernels take a call.  Both the one-step and the multi-step entry point ask this, and neither the answer
+// nor the order of the sums depends on the alignment of q, k and v, so that their results agree bit for bit.
+bool strip_fits(int key_dim, int value_dim, const float* state, const float* new_state) {
     const uintptr_t st = reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(new_state);
-    return value_dim % 4 == 0 && key_dim % 4 == 0 && key_dim <= 256 && (qkv & quad) == 0 && (st & 15u) == 0;
+    return value_dim % 4 == 0 && key_dim % 4 == 0 && key_dim <= 256 && (st & 15u) == 0;
+}
+template <typename T>
+bool quads_aligned(const void* q, const void* k, const void* v) {
+    return ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & (4 * sizeof(T) - 1)) == 0;
 }
 
 template <typename T>
-int launch_linear(const LinParams& p, int dtype, cudaStream_t stream) {
+int launch_linear(const LinParams& p, cudaStream_t stream) {
     const int slices = (p.Dv + kLinCols - 1) / kLinCols;
     const long long ctas = (long long)p.B * p.Hv * slices;
     if (ctas > 0x7fffffffLL) MK36_FAIL(MK36_ERR_UNSUPPORTED, "linear_attention_decode: too many (batch, head) pairs");
     const size_t smem = (size_t)2 * p.Dk * sizeof(float);
     if (smem > 40 * 1024) MK36_FAIL(MK36_ERR_UNSUPPORTED, "linear_attention_decode: key_dim %d is too large", p.Dk);
-    if (strip_fits(dtype, p.Dk, p.Dv, p.q, p.k, p.v, p.state, p.new_state)) {
-        if (p.Dk == 128) linear_strip_kernel<T, 4, true><<<(unsigned)ctas, kStripThreads, smem, stream>>>(p);
-        else if (p.Dk < 128) linear_strip_kernel<T, 4, false><<<(unsigned)ctas, kStripThreads, smem, stream>>>(p);
-        else linear_strip_kernel<T, 8, false><<<(unsigned)ctas, kStripThreads, smem, stream>>>(p);
+    if (strip_fits(p.Dk, p.Dv, p.state, p.new_state)) {
+        const bool aligned = quads_aligned<T>(p.q, p.k, p.v);
+        if (!aligned && p.Dk <= 128) linear_strip_kernel<T, 4, false, false><<<(unsigned)ctas, kStripThreads, smem, stream>>>(p);
+        else if (!aligned) linear_strip_kernel<T, 8, false, false><<<(unsigned)ctas, kStripThreads, smem, stream>>>(p);
+        else if (p.Dk == 128) linear_strip_kernel<T, 4, true, true><<<(unsigned)ctas, kStripThreads, smem, stream>>>(p);
+        else if (p.Dk < 128) linear_strip_kernel<T, 4, false, true><<<(unsigned)ctas, kStripThreads, smem, stream>>>(p);
+        else linear_strip_kernel<T, 8, false, true><<<(unsigned)ctas, kStripThreads, smem, stream>>>(p);
         MK36_CUDA_OK(cudaGetLastError());
         return MK36_OK;
     }
-    // key_dim above 256 or not a multiple of four, or unaligned tensors
+    // key_dim above 256, a dimension that is not a multiple of four, or an unaligned state
     const bool vec = (p.Dv % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.state) & 15u) == 0) &&
                      ((reinterpret_cast<uintptr_t>(p.new_state) & 15u) == 0);
     if (vec) linear_attention_kernel<T, 4><<<(unsigned)ctas, kLinThreads, smem, stream>>>(p);
@@ -473,11 +616,18 @@ int launch_linear(const LinParams& p, int dtype, cudaStream_t stream) {
 }
 
 template <typename T>
-void launch_strip_steps(const LinStepsParams& p, unsigned ctas, cudaStream_t stream) {
+void launch_steps(const LinStepsParams& p, bool strip, unsigned ctas, cudaStream_t stream) {
+    if (!strip) {
+        linear_attention_steps_kernel<T><<<ctas, kLinThreads, (size_t)2 * p.Dk * sizeof(float), stream>>>(p);
+        return;
+    }
     const size_t smem = (size_t)(kStripAhead + 1) * kStripChunk * strip_step_bytes(p.Dk, sizeof(T));  // at most 35 KB
-    if (p.Dk == 128) linear_strip_steps_kernel<T, 4, true><<<ctas, kStripThreads, smem, stream>>>(p);
-    else if (p.Dk < 128) linear_strip_steps_kernel<T, 4, false><<<ctas, kStripThreads, smem, stream>>>(p);
-    else linear_strip_steps_kernel<T, 8, false><<<ctas, kStripThreads, smem, stream>>>(p);
+    const bool aligned = quads_aligned<T>(p.q, p.k, p.v);
+    if (!aligned && p.Dk <= 128) linear_strip_steps_kernel<T, 4, false, false><<<ctas, kStripThreads, smem, stream>>>(p);
+    else if (!aligned) linear_strip_steps_kernel<T, 8, false, false><<<ctas, kStripThreads, smem, stream>>>(p);
+    else if (p.Dk == 128) linear_strip_steps_kernel<T, 4, true, true><<<ctas, kStripThreads, smem, stream>>>(p);
+    else if (p.Dk < 128) linear_strip_steps_kernel<T, 4, false, true><<<ctas, kStripThreads, smem, stream>>>(p);
+    else linear_strip_steps_kernel<T, 8, false, true><<<ctas, kStripThreads, smem, stream>>>(p);
 }
 
 }  // namespace mk36
@@ -510,15 +660,16 @@ extern "C" int mk36_linear_attention_decode(const mk36_linear_attention_args* a,
     p.decay = a->decay;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     switch (a->dtype) {
-        case MK36_BF16: return launch_linear<__nv_bfloat16>(p, a->dtype, s);
-        case MK36_F16: return launch_linear<__half>(p, a->dtype, s);
-        case MK36_F32: return launch_linear<float>(p, a->dtype, s);
+        case MK36_BF16: return launch_linear<__nv_bfloat16>(p, s);
+        case MK36_F16: return launch_linear<__half>(p, s);
+        case MK36_F32: return launch_linear<float>(p, s);
         default: MK36_FAIL(MK36_ERR_UNSUPPORTED, "linear_attention_decode: unsupported dtype %d", a->dtype);
     }
 }
 
-// Several steps in one call; see the strip kernel above.  Calls that it does not take (strip_fits) run the
-// single-step kernel once per step on the same stream, with the same results.
+// Several steps in one call: the strips, else the state in registers all the same.  What remains (value_dim not a multiple
+// of four, key_dim above 256, an unaligned state) runs the single-step kernel once per step on the same stream, with the
+// same results.
 extern "C" int mk36_linear_attention_decode_steps(const mk36_linear_attention_steps_args* a, void* stream) {
     if (!a) MK36_FAIL(MK36_ERR_INVALID_ARG, "linear_attention_decode_steps: args is NULL");
     if (!a->q || !a->k || !a->v || !a->state || !a->out || !a->new_state)
@@ -531,9 +682,11 @@ extern "C" int mk36_linear_attention_decode_steps(const mk36_linear_attention_st
         MK36_FAIL(MK36_ERR_UNSUPPORTED, "linear_attention_decode_steps: unsupported dtype %d", a->dtype);
     if (!current_device_info()) return MK36_ERR_LAUNCH;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const bool fast = strip_fits(a->dtype, a->key_dim, a->value_dim, a->q, a->k, a->v, a->state, a->new_state);
+    const bool strip = strip_fits(a->key_dim, a->value_dim, a->state, a->new_state);
+    const bool resident = a->value_dim % 4 == 0 && a->key_dim <= kLinStepRows * 32 &&
+                          ((reinterpret_cast<uintptr_t>(a->state) | reinterpret_cast<uintptr_t>(a->new_state)) & 15u) == 0;
     const size_t es = a->dtype == MK36_F32 ? 4 : 2;
-    if (!fast) {
+    if (!resident) {
         const size_t qk = (size_t)a->batch * a->key_heads * a->key_dim * es, vb = (size_t)a->batch * a->value_heads * a->value_dim * es;
         const size_t gs = (size_t)a->batch * a->value_heads;
         for (int t = 0; t < a->steps; ++t) {
@@ -568,9 +721,9 @@ extern "C" int mk36_linear_attention_decode_steps(const mk36_linear_attention_st
     const long long ctas = (long long)p.B * p.Hv * ((p.Dv + kStripCols - 1) / kStripCols);
     if (ctas > 0x7fffffffLL) MK36_FAIL(MK36_ERR_UNSUPPORTED, "linear_attention_decode_steps: too many (batch, head) pairs");
     switch (a->dtype) {
-        case MK36_BF16: launch_strip_steps<__nv_bfloat16>(p, (unsigned)ctas, s); break;
-        case MK36_F16: launch_strip_steps<__half>(p, (unsigned)ctas, s); break;
-        default: launch_strip_steps<float>(p, (unsigned)ctas, s); break;
+        case MK36_BF16: launch_steps<__nv_bfloat16>(p, strip, (unsigned)ctas, s); break;
+        case MK36_F16: launch_steps<__half>(p, strip, (unsigned)ctas, s); break;
+        default: launch_steps<float>(p, strip, (unsigned)ctas, s); break;
     }
     MK36_CUDA_OK(cudaGetLastError());
     return MK36_OK;

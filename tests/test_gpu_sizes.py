@@ -210,3 +210,52 @@ def test_moe_wide_kernel_keeps_infinite_weights(cuda_device):
     assert bool(want[:, rows].isinf().all())
     assert torch.equal(got[:, rows], want[:, rows])
     assert_output_parity(got[:, 1::2].cpu(), want[:, 1::2].cpu(), what="rows without an infinite weight")
+
+
+def _graph_nodes(call):
+    """How many nodes a call leaves in a CUDA graph: its launches."""
+    import ctypes
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    count = ctypes.c_size_t()
+    assert ctypes.CDLL("libcudart.so.12").cudaGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(count)) == 0
+    return count.value
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "f16", "f32"])
+@pytest.mark.parametrize("key_dim,value_dim,steps,offset", [(6, 8, 3, 0), (126, 36, 5, 0), (130, 32, 4, 1), (128, 128, 6, 1), (36, 20, 9, 3), (256, 32, 2, 1), (64, 64, 5, 2)])
+def test_linear_attention_steps_keep_the_state_on_chip_for_odd_and_unaligned_inputs(key_dim, value_dim, steps, offset, dtype, cuda_device):
+    """Key dimensions that are no multiple of four, and q, k, v that start `offset` elements off an aligned address: one
+    launch for all steps, the state bit-equal to the oracle's, the outputs to those of one-step calls on aligned tensors."""
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import synthetic as syn
+    from oracle import decode_oracle as oracle
+
+    B, HK, HV = 2, 2, 4
+    stream = list(syn.linear_step_stream(B, HK, HV, key_dim, value_dim, steps=steps, seed=key_dim + steps, dtype=dtype))
+
+    def shifted(name):
+        t = torch.stack([s[name] for s in stream])
+        buf = torch.zeros(t.numel() + 8, dtype=dtype, device=cuda_device)
+        buf[offset:offset + t.numel()] = t.flatten().to(cuda_device)
+        return buf[offset:offset + t.numel()].view(t.shape)
+
+    q, k, v = (shifted(n) for n in ("q", "k", "v"))
+    g, beta = (torch.stack([s[n] for s in stream]).to(cuda_device) for n in ("g", "beta"))
+    s_ref = syn.linear_state(B, HV, key_dim, value_dim, seed=3)
+    state = s_ref.to(cuda_device)
+    run = lambda: mk.linear_attention_decode_steps(q, k, v, state, decay_per_step=g, beta_per_step=beta)
+    outs, final = run()
+    s_one = state
+    for i, step in enumerate(stream):
+        o_ref, s_ref = oracle.linear_attention_decode_per_head(step["q"], step["k"], step["v"], s_ref, step["g"], step["beta"])
+        o_one, s_one = mk.linear_attention_decode_gated(q[i].clone(), k[i].clone(), v[i].clone(), s_one, decay_per_head=g[i], beta_per_head=beta[i])
+        o_off, _ = mk.linear_attention_decode_gated(q[i], k[i], v[i], state if i == 0 else s_prev, decay_per_head=g[i], beta_per_head=beta[i])
+        s_prev = s_one
+        assert torch.equal(s_one.cpu(), s_ref)
+        assert torch.equal(outs[i], o_one) and torch.equal(o_off, o_one)
+        assert_output_parity(outs[i].cpu(), o_ref, what=f"steps {key_dim}x{value_dim}+{offset} out {i}")
+    assert torch.equal(final, s_one)
+    assert _graph_nodes(run) == 1
