@@ -64,8 +64,15 @@ __device__ __forceinline__ void split_hi_lo(const float4& a, const float4& b, ui
     lo = *reinterpret_cast<const uint4*>(l);
 }
 
+// Output row `row` of a token whose down product came out as an infinity or NaN, from the activations' values.
 template <typename T>
-__global__ void __launch_bounds__(kDenseThreads, 1) dense_ffn_mma_kernel(const DenseMmaParams p) {
+static __device__ __noinline__ float dense_mma_again(const DenseMmaParams& p, int token, int row) {
+    const float* act = p.act + token * (size_t)p.I;
+    return down_element_again(static_cast<const T*>(p.down) + (size_t)row * p.I, p.I, [=](int k) { return __ldcg(act + k); });
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kDenseThreads, 1) dense_ffn_mma_kernel(const __grid_constant__ DenseMmaParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_flag;
     __shared__ unsigned s_step;
@@ -298,6 +305,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) dense_ffn_mma_kernel(const D
         float v = 0.0f;
 #pragma unroll
         for (int w = 0; w < kDenseWarps; ++w) v += red[((size_t)w * kDenseMaxTiles + tile) * 128 + rr * 8 + c];
+        if (!(fabsf(v) < INFINITY)) v = dense_mma_again<T>(p, c, h0 + r);
         const size_t o = (size_t)c * H + h0 + r;
         if (exchange) {
             comm_put(p.comm, step, o, v);

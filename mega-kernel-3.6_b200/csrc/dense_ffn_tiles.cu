@@ -53,6 +53,7 @@ struct DenseTilesParams {
     Control* ctl;
     void* act_hi;  // [8][I] in the storage dtype: silu(g) * u = hi + lo
     void* act_lo;
+    float* act;    // [8][I]: silu(g) * u where hi is not finite (f16 ends at 65504), unwritten elsewhere
     int ntok, H, I, add_residual;
     float eps;
     int pa, kca;   // phase A: channels per tile, columns per stage
@@ -61,8 +62,21 @@ struct DenseTilesParams {
     CommParams comm;
 };
 
+// Output row `row` of a token whose down product came out as an infinity or NaN, from the activations' values.
 template <typename T>
-__global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const DenseTilesParams p) {
+static __device__ __noinline__ float dense_tiles_again(const DenseTilesParams& p, int token, int row) {
+    const size_t I = (size_t)p.I;
+    const T* hi = static_cast<const T*>(p.act_hi) + token * I;
+    const T* lo = static_cast<const T*>(p.act_lo) + token * I;
+    const float* whole = p.act + token * I;
+    return down_element_again(static_cast<const T*>(p.down) + (size_t)row * I, p.I, [=](int k) {
+        const float h = to_float<T>(__ldcg(hi + k));
+        return fabsf(h) < INFINITY ? h + to_float<T>(__ldcg(lo + k)) : __ldcg(whole + k);
+    });
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const __grid_constant__ DenseTilesParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int s_flag;
     __shared__ int s_abort;
@@ -255,8 +269,11 @@ __global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const De
                 }
                 const float v = silu(gv) * uv;
                 const T hi = from_float<T>(v);
-                act_hi[(size_t)tok * I + first + ch] = hi;
-                act_lo[(size_t)tok * I + first + ch] = from_float<T>(v - to_float<T>(hi));
+                const bool fits = fabsf(to_float<T>(hi)) < INFINITY;
+                const size_t at = (size_t)tok * I + first + ch;
+                act_hi[at] = hi;
+                act_lo[at] = from_float<T>(fits ? v - to_float<T>(hi) : 0.0f);
+                if (!fits) p.act[at] = v;
             }
         }
         buffer ^= 1;
@@ -359,6 +376,7 @@ __global__ void __launch_bounds__(kDtThreads, 1) dense_ffn_tiles_kernel(const De
         float v = 0.0f;
 #pragma unroll
         for (int w = 0; w < kDtWarps; ++w) v += red[(w * kDtMaxTiles + tile) * 128 + rr * 8 + c];
+        if (!(fabsf(v) < INFINITY)) v = dense_tiles_again<T>(p, c, h0 + r);
         const size_t o = (size_t)c * H + h0 + r;
         if (exchange) {
             comm_put(p.comm, step, o, v);
@@ -428,11 +446,11 @@ int dense_ffn_tiles_launch(const mk36_dense_ffn_args* a, const mk36_comm* comm, 
     if (rc != MK36_OK) return rc;
     if (p.comm.world > 1 && (!a->out || a->partial_out))
         MK36_FAIL(MK36_ERR_INVALID_ARG, "dense_ffn_decode: the multi-GPU entry point writes `out` and takes no partial_out");
+    // a smaller workspace takes the register-staged kernel, which needs half of it; scratch ends below the mailboxes
     const size_t act_bytes = align_up((size_t)kDtMaxTokens * I * 2, 256);
-    if (!workspace || reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
-        MK36_FAIL(MK36_ERR_WORKSPACE, "dense_ffn_decode: workspace is NULL or not 256-byte aligned");
-    if (workspace_bytes < kControlBytes + 2 * act_bytes)
-        MK36_FAIL(MK36_ERR_WORKSPACE, "dense_ffn_decode: workspace too small (%zu < %zu bytes)", workspace_bytes, kControlBytes + 2 * act_bytes);
+    if (!workspace || reinterpret_cast<uintptr_t>(workspace) % 256 != 0 || workspace_bytes < kControlBytes + 4 * act_bytes ||
+        kControlBytes + 4 * act_bytes > kMailboxOffset)
+        return MK36_OK;
 
     p.norm_w = a->norm_weight;
     p.gate = a->gate_weight;
@@ -441,6 +459,7 @@ int dense_ffn_tiles_launch(const mk36_dense_ffn_args* a, const mk36_comm* comm, 
     p.ctl = static_cast<Control*>(workspace);
     p.act_hi = static_cast<unsigned char*>(workspace) + kControlBytes;
     p.act_lo = static_cast<unsigned char*>(workspace) + kControlBytes + act_bytes;
+    p.act = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + kControlBytes + 2 * act_bytes);
     p.H = H;
     p.I = I;
     p.add_residual = a->add_residual;

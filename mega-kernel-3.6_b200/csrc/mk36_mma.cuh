@@ -44,6 +44,24 @@ __device__ __forceinline__ void add_tile(float (&a)[4], const float (&b)[4]) {
     for (int i = 0; i < 4; ++i) a[i] += b[i];
 }
 
+// A down element once more as a plain sum, for one that came out as an infinity or NaN of a product with activations split
+// into high and low halves: a half may be infinite where the fp32 value is not (f16 ends at 65504), and an infinite weight
+// times a half that is zero is a NaN.  `act(c)`: the fp32 activation of channel c.  n is a multiple of eight.
+template <typename T, typename Act>
+__device__ __forceinline__ float down_element_again(const T* w, int n, Act act) {
+    float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int c = 0; c < n; c += 8) {
+        Chunk8<T> v;
+        v.raw = *reinterpret_cast<const uint4*>(w + c);
+        float f[8];
+        unpack8(v, f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum[i] = fmaf(act(c + i), f[i], sum[i]);
+    }
+    return ((sum[0] + sum[1]) + (sum[2] + sum[3])) + ((sum[4] + sum[5]) + (sum[6] + sum[7]));
+}
+
 #endif  // __CUDACC__
 
 }  // namespace mk36

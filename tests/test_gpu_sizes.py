@@ -259,3 +259,36 @@ def test_linear_attention_steps_keep_the_state_on_chip_for_odd_and_unaligned_inp
         assert_output_parity(outs[i].cpu(), o_ref, what=f"steps {key_dim}x{value_dim}+{offset} out {i}")
     assert torch.equal(final, s_one)
     assert _graph_nodes(run) == 1
+
+
+@pytest.mark.parametrize("tiles", [1, 0], ids=["tiles", "register_staged"])
+@pytest.mark.parametrize("what", ["f16_activation_beyond_f16", "infinite_weight"])
+def test_dense_tensor_core_kernels_where_a_split_activation_is_not_finite(what, tiles, cuda_device):
+    """The activations are multiplied as a high and a low half.  One that f16 cannot hold must still give the oracle's finite
+    output, and an infinite down weight an infinity of the activation's sign, as with one token, where nothing is split."""
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import cabi, synthetic as syn
+    from oracle import decode_oracle as oracle
+
+    dtype = torch.float16 if what.startswith("f16") else torch.bfloat16
+    t = syn.dense_tensors(syn.DenseShape(2400, 1216), 1, 5, dtype)
+    t["x"] = t["x"].repeat(5, 1).contiguous()
+    rows = torch.arange(0, 2400, 2)
+    if what.startswith("f16"):
+        for name in ("gate_weight", "up_weight"):
+            t[name][7] = (t["x"][0].float().sign() * 2.0).to(dtype)  # about 3800 each, 1.5e7 as a product
+        t["down_weight"][:, 7] = (t["down_weight"][:, 7].float() * 1e-3).to(dtype)
+    else:
+        t["down_weight"][rows, (rows * 7) % 1216] = float("inf")
+    d = {k: v.to(cuda_device) for k, v in t.items()}
+    weights = mk.DenseFfnWeights(*[d[f] for f in syn.DENSE_WEIGHT_FIELDS])
+    cabi.check(cabi.load().mk36_set_option(b"dense_tiles", tiles))
+    try:
+        got = mk.dense_ffn_decode(d["x"], weights).cpu()
+    finally:
+        cabi.check(cabi.load().mk36_set_option(b"dense_tiles", 1))
+    want = oracle.dense_ffn_decode(t["x"], *[t[f] for f in syn.DENSE_WEIGHT_FIELDS])
+    if not what.startswith("f16"):
+        assert bool(want[:, rows].isinf().all()) and torch.equal(got[:, rows], want[:, rows])
+        got, want = got[:, 1::2], want[:, 1::2]
+    assert_output_parity(got, want, what=f"{what} tiles={tiles}")
