@@ -262,12 +262,13 @@ def attention_block_decode(hidden: torch.Tensor, block: AttentionBlockInputs, *,
     if (
         block.input_norm_weight is not None and k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.shape == v_cache.shape == (b, k_cache.shape[1], hkv, d)
         and hidden.dtype == k_cache.dtype == v_cache.dtype and hidden.device == k_cache.device == v_cache.device
-        and (cos is None or (cos.numel() == sin.numel() == cos.shape[-1] == sin.shape[-1] == block.rotary_dim <= d))
+        # one row of cos and sin; scalars and tables that broadcast some other way take the steps below
+        and (cos is None or (1 <= cos.ndim <= 3 and 1 <= sin.ndim <= 3 and cos.numel() == sin.numel() == cos.shape[-1] == sin.shape[-1] == block.rotary_dim <= d))
     ):
         ext = _native("attention_block_decode", hidden, k_cache, v_cache, block.qkv_weight, block.out_weight, block.input_norm_weight)
         if cos is not None:
-            cos = cos.to(device=hidden.device, dtype=torch.float32).reshape(-1)
-            sin = sin.to(device=hidden.device, dtype=torch.float32).reshape(-1)
+            cos = cos.to(device=hidden.device, dtype=torch.float32).reshape(-1).contiguous()
+            sin = sin.to(device=hidden.device, dtype=torch.float32).reshape(-1).contiguous()
         scale = 1.0 / math.sqrt(d) if block.scale is None else block.scale
         return ext.attention_block_decode(hidden, block.input_norm_weight, block.qkv_weight, block.out_weight, k_cache, v_cache,
                                           block.position, hq, hkv, d, cos, sin, float(scale), float(eps))

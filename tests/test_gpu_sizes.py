@@ -292,3 +292,31 @@ def test_dense_tensor_core_kernels_where_a_split_activation_is_not_finite(what, 
         assert bool(want[:, rows].isinf().all()) and torch.equal(got[:, rows], want[:, rows])
         got, want = got[:, 1::2], want[:, 1::2]
     assert_output_parity(got, want, what=f"{what} tiles={tiles}")
+
+
+@pytest.mark.parametrize("form", ["strided", "expanded", "row_of_three_dimensions", "float64_on_the_host", "scalar"])
+def test_attention_block_takes_cos_and_sin_as_tensor_operations_do(form, cuda_device):
+    """cos and sin that are views with strides, leading dimensions, another type or device, or scalars give what their plain
+    form gives."""
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import synthetic as syn
+
+    hq, hkv, d, B, H, rotary = 4, 2, 64, 2, 256, 32
+    qkv = syn.projection_tensors(H, (hq + 2 * hkv) * d, B, seed=1, norm=True, residual=False)
+    outp = syn.projection_tensors(hq * d, H, B, seed=2, norm=False, residual=False)
+    ang = torch.arange(rotary // 2, dtype=torch.float32) * 0.3 + 0.2
+    cos, sin = ang.cos().repeat(2).to(cuda_device), ang.sin().repeat(2).to(cuda_device)
+    if form in ("expanded", "scalar"):
+        cos, sin = torch.full_like(cos, 0.6), torch.full_like(sin, 0.8)
+    change = {"strided": lambda t: torch.stack((t, -t), dim=1)[:, 0], "expanded": lambda t: t[:1].expand(rotary),
+              "row_of_three_dimensions": lambda t: t.view(1, 1, rotary), "float64_on_the_host": lambda t: t.double().cpu(), "scalar": lambda t: t[0]}[form]
+
+    def run(c, s):
+        cache = {n: t.to(cuda_device) for n, t in syn.attention_tensors(B, hq, hkv, d, 20, seed=3).items()}
+        block = mk.AttentionBlockInputs(qkv["norm_weight"].to(cuda_device), qkv["weight"].to(cuda_device), outp["weight"].to(cuda_device), cache["k_cache"],
+                                        cache["v_cache"], 11, hq, hkv, d, cos=c, sin=s, rotary_dim=rotary)
+        out, attn = mk.attention_block_decode(qkv["x"].to(cuda_device), block)
+        return out, attn, cache["k_cache"]
+
+    for got, want in zip(run(change(cos), change(sin)), run(cos, sin)):
+        assert_output_parity(got.cpu(), want.cpu(), what=f"cos and sin {form}")
