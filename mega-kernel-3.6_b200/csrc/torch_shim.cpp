@@ -450,6 +450,9 @@ std::tuple<torch::Tensor, torch::Tensor> attention_block_decode(torch::Tensor hi
     ap.position = position;
     ap.capacity = k_cache.size(1);
     const auto stream = at::cuda::getCurrentCUDAStream().stream();
+    // the caches are written behind autograd's back: their version counters still have to move, as with any in-place operation
+    k_cache.unsafeGetTensorImpl()->bump_version();
+    v_cache.unsafeGetTensorImpl()->bump_version();
     check_rc(mk36_attention_append(&ap, stream));
     mk36_attention_args a{};
     a.q = ap.q;

@@ -297,7 +297,7 @@ def test_dense_tensor_core_kernels_where_a_split_activation_is_not_finite(what, 
 @pytest.mark.parametrize("form", ["strided", "expanded", "row_of_three_dimensions", "float64_on_the_host", "scalar"])
 def test_attention_block_takes_cos_and_sin_as_tensor_operations_do(form, cuda_device):
     """cos and sin that are views with strides, leading dimensions, another type or device, or scalars give what their plain
-    form gives."""
+    form gives, and the caches' version counters move as with any in-place operation."""
     import mega_kernel_qwen36 as mk
     from mega_kernel_qwen36 import synthetic as syn
 
@@ -315,7 +315,9 @@ def test_attention_block_takes_cos_and_sin_as_tensor_operations_do(form, cuda_de
         cache = {n: t.to(cuda_device) for n, t in syn.attention_tensors(B, hq, hkv, d, 20, seed=3).items()}
         block = mk.AttentionBlockInputs(qkv["norm_weight"].to(cuda_device), qkv["weight"].to(cuda_device), outp["weight"].to(cuda_device), cache["k_cache"],
                                         cache["v_cache"], 11, hq, hkv, d, cos=c, sin=s, rotary_dim=rotary)
+        before = cache["k_cache"]._version, cache["v_cache"]._version
         out, attn = mk.attention_block_decode(qkv["x"].to(cuda_device), block)
+        assert cache["k_cache"]._version > before[0] and cache["v_cache"]._version > before[1]
         return out, attn, cache["k_cache"]
 
     for got, want in zip(run(change(cos), change(sin)), run(cos, sin)):
