@@ -447,16 +447,18 @@ def build_qwen36_decode_tgraph(
 # ---------------------------------------------------------------------------------------------
 # Launch geometry of the kernels in csrc/: threads per CTA, grid-wide barriers per launch.  The numbers
 # mirror the constants of the .cu files (kStThreads, kRingThreads, kDenseThreads, kMmaAttnThreads,
-# kLinThreads, kDsThreads, kAsThreads); tests/test_host_api.py reads those files and fails when the two drift apart.
+# kLinThreads, kDsThreads, kAsThreads, kDtThreads, kStripThreads, kWdThreads); tests/test_host_api.py reads those files and fails when the two drift apart.
 KERNEL_GEOMETRY = {
     "moe_decode_stream_kernel": {"block": 416, "grid_barriers": 1, "max_tokens": 1},
     "moe_decode_batch_kernel": {"block": 416, "grid_barriers": 1, "max_tokens": 8},
+    "moe_decode_wide_kernel": {"block": 384, "grid_barriers": 2, "max_tokens": 32, "fewest_tokens": 9},
     "moe_decode_ring_kernel": {"block": 416, "grid_barriers": 2, "max_tokens": 8},
     "dense_ffn_mma_kernel": {"block": 512, "grid_barriers": 1, "max_tokens": 8},
     "dense_ffn_tiles_kernel": {"block": 288, "grid_barriers": 1, "max_tokens": 8},
+    "attention_append_kernel": {"block": 256, "grid_barriers": 0},
     "attention_decode_stream_kernel": {"block": 288, "grid_barriers": 1},
     "dense_ffn_stream_kernel": {"block": 416, "grid_barriers": 1, "max_tokens": 1},
-    "linear_attention_kernel": {"block": 256, "grid_barriers": 0},  # unaligned shapes only
+    "linear_attention_kernel": {"block": 256, "grid_barriers": 0},  # dimensions that are no multiples of four only
     "linear_strip_kernel": {"block": 64, "grid_barriers": 0},
     "linear_decode_kernel": {"block": 288, "grid_barriers": 0, "max_tokens": 8},
 }
@@ -470,6 +472,20 @@ def moe_batch_kernel_fits(hidden: int, experts: int, top_k: int, intermediate: i
     return (hidden % 256 == 0 and sms <= hidden <= 8 * 384 and intermediate % 32 == 0 and shared_intermediate % 32 == 0
             and 0 < intermediate <= 512 and shared_intermediate <= 512 and 0 < top_k <= 8 and experts <= 256
             and hr_max <= 16 and hr_max * intermediate * 2 <= _RING_STAGE and (-(-experts // sms) + 1) * 8 <= 24)
+
+
+def moe_wide_kernel_fits(hidden: int, experts: int, top_k: int, intermediate: int, shared_intermediate: int, sms: int = 148) -> bool:
+    """Shape conditions of the launcher in csrc/moe_decode_wide.cu (bf16); its shared memory holds 32 tokens of any of them."""
+    return (hidden % 1024 == 0 and 0 < hidden <= 2048 and intermediate % 256 == 0 and shared_intermediate % 256 == 0 and intermediate > 0
+            and 0 < top_k <= 8 and 0 < experts <= 256 and -(-hidden // sms) <= 16 and -(-experts // sms) <= 2
+            and 256 * 3 * intermediate * 2 + 32 * 3 * shared_intermediate * 2 <= 15 << 20)
+
+
+def dense_tiles_kernel_fits(hidden: int, intermediate: int, sms: int = 148) -> bool:
+    """Shape conditions of the launcher in csrc/dense_ffn_tiles.cu: three stages beside the eight tokens, a tile per CTA in
+    both phases and at most three tiles of output rows."""
+    return (hidden % 32 == 0 and intermediate % 32 == 0 and min(hidden, intermediate) >= sms and -(-hidden // sms) <= 48
+            and _SMEM_OPTIN - 1024 - 128 - 8192 - max(16 * (hidden + 8), 8 * 3 * 128 * 4) - 128 >= 3 * 33024)
 
 
 def moe_ring_tokens_per_launch(hidden: int, top_k: int, intermediate: int, shared_intermediate: int, sms: int = 148) -> int:
@@ -512,7 +528,9 @@ def _kernel_schedule(graph: TaskGraph, wc: WorkerConfig, batch: int, context_len
 
     def projection_launch(name: str, group, n_in: int, n_out: int, norm: bool, residual: bool, argmax: bool) -> KernelLaunch:
         geo = KERNEL_GEOMETRY["linear_decode_kernel"]
-        rows = max(1, _RING_STAGE // (n_in * 2))
+        # three to eight tokens on tensor-core tiles: contiguous rows per CTA; else chunks of whole rows
+        tiles = min(batch, geo["max_tokens"]) >= 3 and n_in % 256 == 0
+        rows = 1 if tiles else max(1, _RING_STAGE // (n_in * 2))
         chunks = _ceil_div(n_out, rows)
         phases = ((KernelPhase("rmsnorm_to_smem", 0, 0, "static"),) if norm else ()) + (
             KernelPhase("weight_rows" + ("_residual" if residual else "") + ("_argmax" if argmax else ""), n_out, n_in * 2, "static"),)
@@ -526,6 +544,12 @@ def _kernel_schedule(graph: TaskGraph, wc: WorkerConfig, batch: int, context_len
         if task.kind == "paged_attention":
             hq, hkv, hd = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
             row = hkv * hd * 2
+            # the rotary embedding and the cache append in front of attention; the graph has no task for them
+            heads = hq + 2 * hkv
+            launches.append(KernelLaunch(
+                name=f"layer_{li}_attention_append", entry_point="mk36_attention_append", task_ids=(), kernel="attention_append_kernel",
+                grid=batch * heads, block=min(KERNEL_GEOMETRY["attention_append_kernel"]["block"], _ceil_div(hd, 32) * 32), grid_barriers=0, layer=li,
+                phases=(KernelPhase("rotary_and_append", batch * heads, hd * 2, "static"),), hbm_bytes=2 * batch * heads * hd * 2))
             launches.append(KernelLaunch(
                 name=f"layer_{li}_attention", entry_point="mk36_full_attention_decode", task_ids=(task.id,),
                 kernel="attention_decode_stream_kernel", grid=sms, block=KERNEL_GEOMETRY["attention_decode_stream_kernel"]["block"],
@@ -574,9 +598,12 @@ def _kernel_schedule(graph: TaskGraph, wc: WorkerConfig, batch: int, context_len
             distinct = min(batch * K, E)
             # one token: the stream kernel; more: the batch kernel, eight tokens per launch (the ring
             # kernel, which takes as many tokens per launch as fit beside its activations, for shapes it refuses);
-            # the schedule is by eights also where the launcher serves nine or more bf16 tokens with the wide kernel
+            # nine or more: the wide kernel, 32 tokens per launch
             if batch <= KERNEL_GEOMETRY["moe_decode_stream_kernel"]["max_tokens"]:
                 kname, n_launches = "moe_decode_stream_kernel", 1
+            elif batch >= KERNEL_GEOMETRY["moe_decode_wide_kernel"]["fewest_tokens"] and moe_wide_kernel_fits(H, E, K, I, Is, sms):
+                kname = "moe_decode_wide_kernel"
+                n_launches = _ceil_div(batch, KERNEL_GEOMETRY[kname]["max_tokens"])
             elif moe_batch_kernel_fits(H, E, K, I, Is, sms):
                 kname = "moe_decode_batch_kernel"
                 n_launches = _ceil_div(batch, KERNEL_GEOMETRY[kname]["max_tokens"])
@@ -598,7 +625,7 @@ def _kernel_schedule(graph: TaskGraph, wc: WorkerConfig, batch: int, context_len
             group = by_layer.pop(li, []) + [task]
             I = cfg.intermediate_size
             # one token streams; more use the tensor cores, fed by a ring where three stages fit beside the tokens
-            ring_fits = _SMEM_OPTIN - 1024 - 128 - 8192 - 16 * (H + 8) >= 3 * 33024 and min(H, I) >= sms
+            ring_fits = dense_tiles_kernel_fits(H, I, sms)
             dense_kernel = "dense_ffn_stream_kernel" if batch == 1 else "dense_ffn_tiles_kernel" if ring_fits else "dense_ffn_mma_kernel"
             launches.append(KernelLaunch(
                 name=f"layer_{li}_dense_ffn", entry_point="mk36_dense_ffn_decode", task_ids=tuple(t.id for t in group),

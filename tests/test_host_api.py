@@ -108,12 +108,26 @@ def test_b200_worker_defaults_and_kernel_schedule():
     assert head.hbm_bytes == syn.projection_algorithmic_bytes(*syn.LM_HEAD_35B, 1, norm=True, residual=False)
     assert (head.kernel, head.block, head.grid_barriers, head.grid) == ("linear_decode_kernel", 288, 0, 148)
     assert by_name["layer_0_attn_norm"].entry_point is None
-    # eight tokens: the batch kernel in one launch; nineteen: three launches
+    # eight tokens: the batch kernel in one launch; nineteen: the wide kernel in one, 33 in two
     plan8 = mk.build_qwen36_decode_tgraph(cfg, batch_size=8, num_layers=1, worker_config=wc).linearize(wc, batch_size=8)
     moe8 = {k.name: k for k in plan8.kernel_schedule}["layer_0_moe"]
     assert (moe8.kernel, moe8.block, moe8.grid_barriers, moe8.launches) == ("moe_decode_batch_kernel", 416, 1, 1)
     plan19 = mk.build_qwen36_decode_tgraph(cfg, batch_size=19, num_layers=1, worker_config=wc).linearize(wc, batch_size=19)
-    assert {k.name: k for k in plan19.kernel_schedule}["layer_0_moe"].launches == 3
+    moe19 = {k.name: k for k in plan19.kernel_schedule}["layer_0_moe"]
+    assert (moe19.kernel, moe19.block, moe19.grid_barriers, moe19.launches) == ("moe_decode_wide_kernel", 384, 2, 1)
+    plan33 = mk.build_qwen36_decode_tgraph(cfg, batch_size=33, num_layers=1, worker_config=wc).linearize(wc, batch_size=33)
+    assert {k.name: k for k in plan33.kernel_schedule}["layer_0_moe"].launches == 2
+    # rotary embedding and cache append are one launch in front of attention; four tokens project on tensor-core tiles,
+    # a row at least per CTA
+    append = launches["layer_3_attention_append"]
+    assert (append.entry_point, append.kernel, append.grid, append.block) == ("mk36_attention_append", "attention_append_kernel", 20, 256)
+    plan4 = mk.build_qwen36_decode_tgraph(cfg, batch_size=4, num_layers=4, worker_config=wc).linearize(wc, batch_size=4)
+    assert {k.name: k for k in plan4.kernel_schedule}["layer_3_qkv_proj"].grid == 148
+    # the dense tiles: three tiles of output rows per CTA at most, whatever room the ring has
+    assert mpk_graph.dense_tiles_kernel_fits(5120, 17408) and mpk_graph.dense_tiles_kernel_fits(7104, 7104)
+    assert not mpk_graph.dense_tiles_kernel_fits(7136, 7136) and not mpk_graph.dense_tiles_kernel_fits(5120, 128)
+    assert mpk_graph.moe_wide_kernel_fits(2048, 256, 8, 512, 512) and mpk_graph.moe_wide_kernel_fits(1024, 8, 2, 256, 0)
+    assert not mpk_graph.moe_wide_kernel_fits(256, 16, 4, 128, 128) and not mpk_graph.moe_wide_kernel_fits(2048, 512, 8, 512, 512)
     # the ring kernel takes as many tokens per launch as its shared memory holds beside the activations
     assert mpk_graph.moe_ring_tokens_per_launch(2048, 8, 512, 512) in (1, 2, 4, 8)
 
@@ -148,6 +162,18 @@ def test_kernel_geometry_table_matches_the_cuda_sources():
     assert geo["moe_decode_ring_kernel"]["max_tokens"] == ring["kRingMaxTokens"]
     assert mpk_graph._RING_STAGE == ring["kRingStageBytes"]
     assert geo["dense_ffn_mma_kernel"]["block"] == constants("dense_ffn_mma.cu")["kDenseThreads"]
+    wide = constants("moe_decode_wide.cu")
+    assert geo["moe_decode_wide_kernel"]["block"] == wide["kWdThreads"]
+    assert geo["moe_decode_wide_kernel"]["max_tokens"] == wide["kWdMaxTokens"]
+    text = (csrc / "moe_decode_wide.cu").read_text()
+    assert text.count("barrier_arrive(p.ctl") + text.count("grid_barrier(p.ctl") == geo["moe_decode_wide_kernel"]["grid_barriers"]
+    assert re.search(r"int moe_wide = %d;" % geo["moe_decode_wide_kernel"]["fewest_tokens"], (csrc / "mk36_common.cuh").read_text())
+    tiles = constants("dense_ffn_tiles.cu")
+    assert geo["dense_ffn_tiles_kernel"]["block"] == tiles["kDtThreads"]
+    assert geo["dense_ffn_tiles_kernel"]["max_tokens"] == tiles["kDtMaxTokens"]
+    assert (tiles["kDtStageBytes"], 16 * tiles["kDtMaxTiles"]) == (33024, 48)
+    assert geo["linear_strip_kernel"]["block"] == constants("linear_attention_decode.cu")["kStripThreads"]
+    assert "__launch_bounds__(%d) attention_append_kernel" % geo["attention_append_kernel"]["block"] in (csrc / "attention_append.cu").read_text()
     assert geo["attention_decode_stream_kernel"]["block"] == constants("attention_decode_stream.cu")["kAsThreads"]
     assert geo["dense_ffn_stream_kernel"]["block"] == constants("dense_ffn_stream.cu")["kDsThreads"]
     assert geo["linear_attention_kernel"]["block"] == constants("linear_attention_decode.cu")["kLinThreads"]
@@ -290,6 +316,7 @@ def test_ctypes_structures_match_the_c_header(tmp_path):
         "mk36_moe_args": cabi.MoeArgs,
         "mk36_dense_ffn_args": cabi.DenseFfnArgs,
         "mk36_attention_args": cabi.AttentionArgs,
+        "mk36_attention_append_args": cabi.AttentionAppendArgs,
         "mk36_linear_attention_args": cabi.LinearAttentionArgs,
         "mk36_linear_attention_steps_args": cabi.LinearAttentionStepsArgs,
         "mk36_comm": cabi.Comm,
