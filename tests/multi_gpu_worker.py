@@ -98,6 +98,7 @@ def main() -> int:
         # ---------------- dense FFN, tensor parallel ----------------
         dense_cases = [
             ("dense_mid_bf16", syn.DenseShape(256, 704), 3, torch.bfloat16),
+            ("dense_tiles_bf16", syn.DenseShape(1024, 2816), 5, torch.bfloat16),  # the ring-fed tiles at every world size
             ("dense_27b_b1", syn.DENSE_27B, 1, torch.bfloat16),
         ]
         for name, shape, batch, dtype in dense_cases:

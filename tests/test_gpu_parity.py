@@ -151,6 +151,8 @@ def test_moe_batch_kernel_variants_match_oracle(name, option, cuda_device):
     ("35b", 8, torch.bfloat16, True),
     ("35b", 9, torch.bfloat16, False),
     ("35b", 19, torch.bfloat16, False),
+    ("35b", 9, torch.float16, False),
+    ("small", 19, torch.float16, False),
 ], ids=lambda v: str(v).replace("torch.", ""))
 def test_moe_batch_kernel_ragged_and_shared_experts(shape, batch, dtype, same, cuda_device):
     """Token counts that do not fill a launch of eight (3, 5, 7), that need a second and third launch
@@ -165,7 +167,7 @@ def test_moe_batch_kernel_ragged_and_shared_experts(shape, batch, dtype, same, c
         t["x"] = t["x"][:1].repeat(batch, 1).contiguous()
     case = Case(f"moe_{shape}_b{batch}", "moe", lambda: None)
     spec = {"tensors": t, "top_k": shp.top_k}
-    got = run_cuda(case, spec, cuda_device)
+    got = _run_with_options(case, spec, cuda_device, "moe_wide=0")  # nine or more bf16 tokens would run the wide kernel
     ref = run_oracle(case, spec)
     assert_indices_exact(got["indices"], ref["indices"])
     torch.testing.assert_close(got["weights"], ref["weights"], atol=1e-5, rtol=1e-4)
@@ -196,7 +198,7 @@ def test_moe_wide_kernel_matches_oracle(batch, same, fewest, cuda_device):
         assert torch.equal(got["out"], got["out"][:1].expand_as(got["out"])), "identical tokens must give identical rows"
 
 
-@pytest.mark.parametrize("batch", [1, 2, 8])
+@pytest.mark.parametrize("batch", [1, 2, 8, 9, 32])
 def test_moe_equal_logits_go_to_the_lowest_expert_index(batch, cuda_device):
     """Router rows e and e + 128 are made identical, and so are rows 5 and 70, so that every logit has a
     bit-equal twin: in the same lane of the selecting warp (e and e + 128) and in another lane (5 and 70).
@@ -226,9 +228,10 @@ def test_moe_equal_logits_go_to_the_lowest_expert_index(batch, cuda_device):
     assert_output_parity(got["out"], ref.to(got["out"].dtype), what="moe with tied logits")
 
 
+@pytest.mark.parametrize("tiles", [1, 0], ids=["tiles", "register_staged"])
 @pytest.mark.parametrize("name", ["dense_mid_f16_b1", "dense_27b_bf16_b1"])
-def test_dense_one_token_through_the_tensor_core_kernel(name, cuda_device):
-    """One-token dense FFN calls run the streaming kernel; the tensor-core kernel that serves larger
+def test_dense_one_token_through_the_tensor_core_kernel(name, tiles, cuda_device):
+    """One-token dense FFN calls run the streaming kernel; the tensor-core kernels that serve larger
     batches must give the same call the same answer within the tolerances."""
     from mega_kernel_qwen36 import cabi
 
@@ -236,10 +239,12 @@ def test_dense_one_token_through_the_tensor_core_kernel(name, cuda_device):
     spec = build_inputs(case)
     lib = cabi.load()
     cabi.check(lib.mk36_set_option(b"dense_stream", 0))
+    cabi.check(lib.mk36_set_option(b"dense_tiles", tiles))
     try:
         got = run_cuda(case, spec, cuda_device)
     finally:
         cabi.check(lib.mk36_set_option(b"dense_stream", 1))
+        cabi.check(lib.mk36_set_option(b"dense_tiles", 1))
     assert_output_parity(got["out"], run_oracle(case, spec)["out"], what=name + " (tensor-core kernel)")
 
 

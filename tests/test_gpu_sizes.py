@@ -322,3 +322,53 @@ def test_attention_block_takes_cos_and_sin_as_tensor_operations_do(form, cuda_de
 
     for got, want in zip(run(change(cos), change(sin)), run(cos, sin)):
         assert_output_parity(got.cpu(), want.cpu(), what=f"cos and sin {form}")
+
+
+@pytest.mark.parametrize("shape,batch", [((1024, 24, 4, 256, 512), 9), ((1024, 40, 8, 512, 0), 12), ((2048, 8, 1, 256, 256), 32)])
+def test_moe_wide_kernel_at_other_shapes(shape, batch, cuda_device):
+    """Hidden 1024, fewer experts than CTAs, top 4 and top 1 (every expert has several entries), a shared expert of another
+    width than the routed ones, and none."""
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import mpk_graph, synthetic as syn
+    from oracle import decode_oracle as oracle
+
+    assert mpk_graph.moe_wide_kernel_fits(*shape)
+    t = syn.moe_tensors(syn.MoeShape(*shape), batch, 60 + batch, torch.bfloat16)
+    out, idx, w = mk.moe_decode(t["x"].to(cuda_device), mk.MoeWeights(*[t[f].to(cuda_device) for f in syn.MOE_WEIGHT_FIELDS]), top_k=shape[2])
+    want, want_idx, want_w = oracle.moe_decode(t["x"], *[t[f] for f in syn.MOE_WEIGHT_FIELDS], top_k=shape[2])
+    assert torch.equal(idx.cpu(), want_idx)
+    torch.testing.assert_close(w.cpu(), want_w, atol=1e-5, rtol=1e-4)
+    assert_output_parity(out.cpu(), want, what=f"wide {shape} b{batch}")
+
+
+def test_moe_wide_kernel_on_slices_of_the_experts(cuda_device):
+    """The fp32 partials of two expert-parallel slices add up to the whole layer."""
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import ops, parallel, synthetic as syn
+    from oracle import decode_oracle as oracle
+
+    t = syn.moe_tensors(syn.MoeShape(2048, 64, 8, 512, 512), 17, 6, torch.bfloat16)
+    full = mk.MoeWeights(*[t[f].to(cuda_device) for f in syn.MOE_WEIGHT_FIELDS])
+    x, total = t["x"].to(cuda_device), 0.0
+    for rank in range(2):
+        shard = parallel.shard_moe_weights(full, rank, 2)
+        part, idx, _ = ops._C.moe_decode_partial(x, *[getattr(shard.weights, f) for f in syn.MOE_WEIGHT_FIELDS], 1e-6, 8, shard.expert_base)
+        total = total + part
+    want, want_idx, _ = oracle.moe_decode(t["x"], *[t[f] for f in syn.MOE_WEIGHT_FIELDS], top_k=8)
+    assert torch.equal(idx.cpu(), want_idx)
+    assert_output_parity((total + x.float()).bfloat16().cpu(), want, what="wide, two expert slices")
+
+
+@pytest.mark.parametrize("batch,n_in,n_out,dtype", [(3, 2304, 5000, torch.bfloat16), (8, 5376, 700, torch.float16), (4, 256, 3, torch.bfloat16)],
+                         ids=lambda v: str(v).replace("torch.", ""))
+def test_projection_tiles_with_a_narrower_last_stage(batch, n_in, n_out, dtype, cuda_device):
+    """Inner dimensions that are no multiple of a stage's columns, and fewer rows than CTAs."""
+    import mega_kernel_qwen36 as mk
+    from mega_kernel_qwen36 import synthetic as syn
+    from oracle import decode_oracle as oracle
+
+    t = syn.projection_tensors(n_in, n_out, batch, seed=n_in, dtype=dtype, norm=True, residual=True)
+    d = {k: v.to(cuda_device) for k, v in t.items()}
+    got = mk.linear_decode(d["x"], d["weight"], norm_weight=d["norm_weight"], residual=d["residual"]).cpu()
+    want = oracle.linear_decode(t["x"], t["weight"], norm_weight=t["norm_weight"], residual=t["residual"])
+    assert_output_parity(got, want, what=f"projection {n_in}->{n_out}")
