@@ -55,7 +55,7 @@ int dense_launch(const mk36_dense_ffn_args* a, const mk36_moe_args* m, const mk3
             if (rc != MK36_OK || handled) return rc;
         }
         // the ring needs room for three stages beside the eight tokens (hidden size up to about 7000) and a tile per CTA;
-        // 27B shape, eight tokens: 134 us with register loads, 114 through the ring
+        // 27B shape, eight tokens: 133 us with register loads, 115 through the ring; an eighth of it 28.3 and 28.3
         if (options().dense_tiles) {
             const int rc = dense_ffn_tiles_launch(a, comm, workspace, workspace_bytes, stream, &handled);
             if (rc != MK36_OK || handled) return rc;

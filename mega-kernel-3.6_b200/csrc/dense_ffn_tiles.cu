@@ -6,7 +6,7 @@
 // The weight stream bounds it (535 MB at hidden 5120, intermediate 17408).  dense_ffn_mma.cu loads the
 // weights into fragments with register loads and stops at 4.0 TB/s: an SM cannot keep enough such loads
 // outstanding.  Here the copy engine keeps four stages of 32 KB in flight per SM and the registers hold
-// only what is being multiplied: eight tokens at that shape 134 -> 114 us (4.7 TB/s), bf16.
+// only what is being multiplied: eight tokens at that shape 133 -> 115 us (4.6 TB/s), bf16.
 //
 //   stage    up to 16 weight rows by up to 1024 columns, one bulk copy per row; rows lie 16 bytes apart
 //            modulo 128, so that the fragment loads (eight rows, four 16-byte pieces) meet all banks

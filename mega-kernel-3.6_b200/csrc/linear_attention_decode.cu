@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kStripThreads) linear_strip_kernel(const LinPa
 // the same pipe time); a CTA is small (32 columns: 2048 warps at eight tokens of 32 heads, 13.8 per SM);
 // q, k, v travel to shared memory by asynchronous copies, kStripAhead chunks of four steps ahead, and are
 // widened as they are read; and the four read-out sums of a chunk go through their shuffles together.
-// Measured at 64 steps, eight tokens, 32 heads of 128 x 128: 59 us (about 34 us of it is the FP32 pipe of an average
+// Measured at 64 steps, eight tokens, 32 heads of 128 x 128: 59 us (about 29 us of it is the FP32 pipe of an average
 // SM, the rest what the busiest scheduler has above the average and its other instructions); the kernel before
 // it, two barriers of 256 threads and a sum through shared memory per step, took 260 us.
 template <typename T, int NQ, bool FULL, bool ALIGNED>

@@ -105,8 +105,9 @@ __device__ __forceinline__ void attention_merge_items(const AttnParams& p, int f
 // The merge for few splits (several batch items share the grid): an item is (batch, head, 128 channels), lane l has
 // channels 4 l .. 4 l + 3, and the partials of up to 32 splits are in flight at once.  With lanes on the splits, as
 // above, a warp would take B * Hq * D / 4 items over the grid's warps in turn, each a round trip to L2
-// (six items of 3001 tokens, 24 heads of 256: 28.8 us with lanes on the splits, 23.2 this way; three of 6000: 26.8 and
-// 24.6; two of 6000, 74 splits, stay with the lanes on the splits).
+// (24 heads of 256, lanes on the splits and this way: 24 splits, six items of 3001 tokens, 29.0 and 23.5 us; 49, three of
+// 6000, 26.7 and 24.7).  64 splits are two rounds of the 32 rows that a lane's registers hold in flight; with more, from
+// two items down, there are few items per warp and the lanes on the splits ask for all of them at once.
 constexpr int kAttnMergeFewSplits = 64;
 template <typename T>
 __device__ __forceinline__ void attention_merge_few_splits(const AttnParams& p, int first, int total_warps, int lane) {

@@ -670,8 +670,8 @@ int moe_decode_launch(const mk36_moe_args* a, const mk36_comm* comm, void* works
             if (rc != MK36_OK || handled) return rc;
         }
         // nine tokens are where the batch kernel needs a second launch, which reads the experts that both halves chose
-        // twice (32 tokens at the 35B shape: 314 us as four launches, 204 as one); up to eight tokens the batch kernel's
-        // ring streams faster than the wide kernel's register loads
+        // twice (35B shape, launches of eight and one launch: nine tokens 109 and 93 us, 16 157 and 139, 32 315 and 205);
+        // up to eight tokens the batch kernel's ring streams faster than the wide kernel's register loads
         if (options().moe_wide > 0 && a->batch >= options().moe_wide && options().moe_batch && !options().ring_mma) {
             rc = moe_decode_wide_launch(a, comm, workspace, workspace_bytes, stream, &handled);
             if (rc != MK36_OK || handled) return rc;

@@ -23,7 +23,8 @@
 // sums too (1.55e-7 and 1.45e-7, 217 and 219 us).
 //
 //   phase 0   every CTA normalises all tokens into shared memory and dots them with its one or two
-//             router rows (fp32 FMA: the choice of experts does not depend on the kernel) | arrive 1
+//             router rows (fp32 FMA, as in the other kernels; the sum of squares of a token is one warp's
+//             chain here, so that a near tie of two logits may still fall differently)     | arrive 1
 //   phase A'  the shared expert's gate/up units (they need no routing)                   | wait 1
 //   select    every CTA: top-k and soft-max per token, list of entries = (expert, up to eight of its
 //             tokens); an expert with more tokens has several entries, which share its weights in L2
